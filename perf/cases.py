@@ -256,17 +256,22 @@ def _prepare_hook(case, seed):
     for p in model.ft_params():
         is_bias = p.dim() == 4 and p.shape[2] == 1
         p.data.copy_(_randn(p.shape, gen, torch.float32) * (0.1 if is_bias else 0.5 / p.shape[2] ** 0.5))
-    B, hidden = case["batch"], case["q_heads"] * 128
     caches, attns = [None] * case["layers"], [l.self_attn for l in model.model.layers]
+    context, new = _hidden_states(case, seed, dtype)
     with torch.no_grad():
-        for lo in range(0, case["context"], 512):               # the context so far, a chunk at a time
-            h = _randn((B, min(512, case["context"] - lo), hidden), gen, dtype)
-            if h.shape[1] > 1:
-                for i, attn in enumerate(attns):
-                    caches[i] = attn(h, caches[i])[1]
-    return {"case": case, "model": model, "attns": attns, "caches": caches,
-            "h": [_randn((B, case["tokens"], hidden), gen, dtype) for _ in attns],
+        for h in context:
+            for i, attn in enumerate(attns):
+                caches[i] = attn(h, caches[i])[1]
+    return {"case": case, "model": model, "attns": attns, "caches": caches, "h": new,
             "lengths": [0 if c is None else c.length for c in caches]}
+
+
+def _hidden_states(case, seed, dtype):
+    """The context so far, a chunk at a time, and the new tokens of every layer."""
+    gen, B, hidden = _gen(seed + (1 << 32)), case["batch"], case["q_heads"] * 128
+    chunks = (min(512, case["context"] - lo) for lo in range(0, case["context"], 512))
+    context = [_randn((B, n, hidden), gen, dtype) for n in chunks if n > 1]
+    return context, [_randn((B, case["tokens"], hidden), gen, dtype) for _ in range(case["layers"])]
 
 
 @torch.no_grad()
@@ -305,6 +310,49 @@ def prepare(case, seed):
 
 def run(state):
     return globals()["_run_" + state["case"]["kind"]](state)
+
+
+# ------------------------------------------------------------------------------------------ the same in 64 bits
+def exact(case, seed):
+    """Where an output depends on which keys a hash picked, or is a code or a score, there is no value in 64 bits: a key
+    whose score is the threshold may go either way. What is left is the hook's dense attention (a prompt, and the
+    layers that attend to every key) and the rows that go into the caches."""
+    if case["kind"] == "load":
+        st = _prepare_load(case, seed)
+        return [None, st["k"].double(), st["v"].double()]
+    if case["kind"] != "hook":
+        return None
+    dtype, B, T, QH, KH = torch_dtype(case["dtype"]), case["batch"], case["tokens"], case["q_heads"], case["kv_heads"]
+    layers = _attention_model(case, _gen(seed), dtype).model.layers
+    context, new = _hidden_states(case, seed, dtype)
+    n, G, outs, rows = sum(h.shape[1] for h in context), QH // KH, [], []
+    angle = torch.arange(n + T, device=DEV, dtype=torch.float64)[:, None] / THETA ** (torch.arange(0, 128, 2, device=DEV, dtype=torch.float64) / 128)
+    cos, sin = angle.cos()[:, None], angle.sin()[:, None]
+
+    def heads(h, linear, rotate):
+        x = (h.double() @ linear.weight.double().T).view(B, h.shape[1], -1, 128)
+        if rotate is None:
+            return x
+        a, b = x[..., :64], x[..., 64:]
+        c, s = cos[rotate:rotate + h.shape[1]], sin[rotate:rotate + h.shape[1]]
+        return torch.cat([a * c - b * s, b * c + a * s], dim=-1)
+
+    for i, layer in enumerate(layers):
+        at = layer.self_attn
+        h = torch.cat(context + [new[i]], dim=1)
+        k, v = heads(h, at.k_proj, 0), heads(h, at.v_proj, None)
+        rows += [k[:, n:], v[:, n:]]
+        if T == 1 and i >= case["fixed"]:
+            outs.append(None)
+            continue
+        q, o = heads(new[i], at.q_proj, n), torch.empty((B, T, QH, 128), device=DEV, dtype=torch.float64)
+        later = torch.arange(n + T, device=DEV)[None] > n + torch.arange(T, device=DEV)[:, None]
+        for b in range(B):
+            for j in range(QH):
+                s = (q[b, :, j] @ k[b, :, j // G].T / 128 ** 0.5).masked_fill_(later, float("-inf"))
+                o[b, :, j] = s.softmax(dim=-1) @ v[b, :, j // G]
+        outs.append(o.view(B, T, QH * 128) @ at.o_proj.weight.double().T)
+    return outs + rows
 
 
 # ------------------------------------------------------------------------------------------ what a pass cannot do without
