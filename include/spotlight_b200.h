@@ -217,6 +217,21 @@ int sl_decode_prepare_ex(const void* d_q, const void* d_k, const void* d_v, int 
                          int64_t code_batch_stride, void* d_k_cache, void* d_v_cache,
                          const sl_kv_layout* kv, int64_t pos, void* stream);
 
+/* RoPE of a prompt's (or its next chunk's) queries and keys and the append of its rows, one launch, bf16:
+ * d_q [B,T,QH,128] -> d_q_rot (same shape), d_k / d_v [B,T,KH,128] -> rows pos .. pos+T-1 of the caches (geometry kv;
+ * list_heads_per_kv_head is not used), keys rotated. d_cos / d_sin [T,128] are the rows of the new positions. Rounding
+ * points as torch's (x * cos, rotate_half(x) * sin and their sum each rounded to bf16).
+ * Replaces check_and_apply_qk_rope (spotlight/modifiers/modify_llama.py:68-80) + KVCache.update (gpu_cache.py:108-118). */
+int sl_rope_append(const void* d_q, const void* d_k, const void* d_v, int dtype, int B, int64_t T, int QH, int KH,
+                   const void* d_cos, const void* d_sin, void* d_q_rot, void* d_k_cache, void* d_v_cache,
+                   const sl_kv_layout* kv, int64_t pos, void* stream);
+/* Causal attention of T new tokens (positions pos .. pos+T-1, d_q [B,T,QH,128] rotated) over the cached rows
+ * 0 .. pos+T-1, query head j reading kv head j / (QH/KH); out [B,T,QH,128]; bf16, fp32 softmax and sums, scale 1/sqrt(128).
+ * Needs 16-byte aligned rows and, for B > 1, a positive batch stride; QH/KH <= 128. A device-side wait that runs out raises
+ * sl_hash_status. Replaces the dense attention of a prompt (spotlight_generation.py:145-147,217-224). */
+int sl_prefill_attn(const void* d_q, const void* d_k_cache, const void* d_v_cache, int dtype, const sl_kv_layout* kv, int B,
+                    int64_t T, int QH, int KH, int64_t pos, void* d_out, void* stream);
+
 /* Hash + sign + pack of many rows (code-cache build at prefill):
  * d_x [B,T,H,128] with batch stride x_batch_stride (elements) -> d_codes [B,T,H,4] with batch
  * stride code_batch_stride (words). Same rounding as sl_decode_prepare. */

@@ -87,6 +87,8 @@ SIGNATURES = {
     "sl_select_emit": (_I, [_P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _I, _I, _I, _P, _I, _P, _P, _Z, _P, _P]),
     "sl_decode_prepare": (_I, [_P, _P, _P, _I, _I, _I, _I, _P, _P, _HP, _HP, _P, _P, _P, _L, _P, _P, _L, _L, _P]),
     "sl_decode_prepare_ex": (_I, [_P, _P, _P, _I, _I, _I, _I, _P, _P, _HP, _HP, _P, _P, _P, _L, _P, _P, _KV, _L, _P]),
+    "sl_rope_append": (_I, [_P, _P, _P, _I, _I, _L, _I, _I, _P, _P, _P, _P, _P, _KV, _L, _P]),
+    "sl_prefill_attn": (_I, [_P, _P, _P, _I, _KV, _I, _L, _I, _I, _L, _P, _P]),
     "sl_hash_encode": (_I, [_P, _L, _I, _I, _L, _I, _HP, _P, _L, _P]),
     "sl_hash_encode_ex": (_I, [_P, _L, _L, _L, _I, _I, _L, _I, _HP, _P, _L, _P]),
     "sl_sparse_attn_workspace_bytes": (_Z, [_I, _I, _I]),

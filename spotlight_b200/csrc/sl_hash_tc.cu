@@ -29,11 +29,12 @@
 // bounded; a wait that runs out raises the library's hash status word, the CTA lets its copies in flight land, frees
 // its TMEM and returns.
 // Same arithmetic as the warp-level kernel in sl_hash_mma.cu up to the order of the fp32 additions.
-#include <cuda.h>
-
 #include "sl_common.cuh"
+#include "sl_tc.cuh"
 
 namespace {
+
+using namespace sltc;
 
 constexpr int TC_EPI_WARPS = 16;                // 4 lane quadrants x 4 column groups
 constexpr int TC_THREADS = (TC_EPI_WARPS + 1) * 32;
@@ -41,7 +42,6 @@ constexpr int TC_TILE = 128;
 constexpr unsigned W1_BYTES = 128 * 256 * 2, W2_BYTES = 256 * 128 * 2, X_BYTES = TC_TILE * 128 * 2;
 constexpr unsigned OFF_W1 = 0, OFF_W2 = W1_BYTES, OFF_X = W1_BYTES + W2_BYTES, OFF_B1 = OFF_X + 2 * X_BYTES,
                    OFF_B2 = OFF_B1 + 512, OFF_LUT = OFF_B2 + 256, OFF_BAR = OFF_LUT + 16384, OFF_MISC = OFF_BAR + 8 * 8, TC_SMEM = OFF_MISC + 16 + 1024;
-constexpr unsigned WAIT_NS = 20000u, WAIT_TRIES = 50000u, WAIT_LIMIT = 1u << 22;
 
 struct HashTcArgs {
     long long T; int H; int B;
@@ -50,12 +50,6 @@ struct HashTcArgs {
     long long tiles_per_b, n_tiles;
     int* status;                                  // mapped host word: 3 = a wait ran out
 };
-
-__device__ __forceinline__ unsigned pack2(float lo, float hi) {      // two fp32 -> two bf16, round to nearest even, one instruction
-    unsigned r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
 
 // sum of two pairs of bf16, each rounded to nearest even once: equal to the fp32 sum rounded to bf16
 __device__ __forceinline__ unsigned add_bf16x2(unsigned x, unsigned y) {
@@ -78,84 +72,6 @@ constexpr unsigned LUT_LO = 99u << 7;       // 2^-28
 __device__ __noinline__ unsigned silu_pair(unsigned y) {
     return (unsigned)silu_bf16((unsigned short)(y & 0xffffu)) | ((unsigned)silu_bf16((unsigned short)(y >> 16)) << 16);
 }
-
-// ---- mbarrier, TMA, tcgen05 in PTX
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Suspends the thread until the phase completes or about `ns` nanoseconds have passed (no spinning on shared memory,
-// which the tensor core is reading its operands from).
-__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity, unsigned ns) {
-    unsigned ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity), "r"(ns) : "memory");
-    return ok != 0;
-}
-// Bounded wait: false when the limit ran out (WAIT_TRIES suspensions of at most WAIT_NS each and a pause between them:
-// about a second) or another thread of the CTA has already given up.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatile int* abort_flag) {
-    for (unsigned i = 0; i < WAIT_TRIES; ++i) {
-        if (mbar_try(bar, parity, WAIT_NS)) return true;
-        if (*abort_flag) return false;
-        __nanosleep(64);
-    }
-    return false;
-}
-__device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap* map, unsigned bar, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(unsigned bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// D[tmem] (+)= A[smem] B[smem]
-__device__ __forceinline__ void mma_ss(unsigned d, unsigned long long adesc, unsigned long long bdesc, unsigned idesc, unsigned acc) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
-}
-// D[tmem] (+)= A[tmem] B[smem]
-__device__ __forceinline__ void mma_ts(unsigned d, unsigned a, unsigned long long bdesc, unsigned idesc, unsigned acc) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                 ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(unsigned taddr, unsigned (&v)[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                   "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-                   "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-                   "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                 : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_st16(unsigned taddr, const unsigned (&v)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-                   "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// Shared-memory matrix descriptor: K-major rows of 128 bytes (64 bf16), 128-byte swizzle, groups of 8 rows
-// 1024 bytes apart. A K step of 16 elements inside a swizzle row advances the start address by 32 bytes.
-__device__ __forceinline__ unsigned long long smem_desc(unsigned addr) {
-    return (unsigned long long)((addr >> 4) & 0x3fffu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-// Instruction descriptor: fp32 accumulators, bf16 A and B, both K-major, M = 128.
-__host__ __device__ constexpr unsigned instr_desc(int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | (8u << 24); }
 
 // byte offset of element (row, k) of a K-major operand: slabs of 64 k, rows of 128 bytes, 16-byte chunks XORed with row % 8
 __device__ __forceinline__ unsigned kmajor_off(int row, int k, int rows) {
@@ -537,22 +453,7 @@ __global__ void __launch_bounds__(L1_THREADS, 1) hash_encode_tc_linear_kernel(co
     if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) != cudaSuccess || qres != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<EncodeTiledFn>(p);
-    }();
-    return fn;
-}
-
-int* g_status_host = nullptr;     // one mapped host word for the process: any device may raise it
+int* g_status_host = nullptr;     // one mapped host word for the process: any device and any of the tensor-core kernels may raise it
 int g_hash_kernel = 0;            // 0 by shape, 1 warp-level kernel only, 2 this kernel whenever it covers the shape
 
 }  // namespace
@@ -567,6 +468,19 @@ extern "C" int sl_profile_tc_timing(unsigned long long* host_out) {
 namespace sl {
 
 void set_hash_kernel(int mode) { g_hash_kernel = mode; }
+
+// The status word as the current device addresses it (null: none to be had).
+int* tc_status_word() {
+    if (!g_status_host) {
+        int* p = nullptr;
+        if (cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        *p = 0;
+        g_status_host = p;
+    }
+    int* d_status = nullptr;
+    if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&d_status), g_status_host, 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return d_status;
+}
 
 // Returns the hash status word (0, or 3 after a device-side wait ran out) and clears it. The caller synchronises first.
 int take_hash_status() {
@@ -590,14 +504,8 @@ int launch_hash_encode_tc(const void* x, long long xs_b, long long xs_tok, long 
     if (xs_tok % 8 != 0 || xs_h % 8 != 0 || (B > 1 && (xs_b % 8 != 0 || xs_b <= 0))) return 1;
     EncodeTiledFn enc = encode_fn();
     if (!enc) return 1;
-    if (!g_status_host) {
-        int* p = nullptr;
-        if (cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return 1; }
-        *p = 0;
-        g_status_host = p;
-    }
-    int* d_status = nullptr;
-    if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&d_status), g_status_host, 0) != cudaSuccess) { cudaGetLastError(); return 1; }
+    int* d_status = sl::tc_status_word();
+    if (!d_status) return 1;
 
     CUtensorMap map;
     const cuuint64_t gdim[4] = {128, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};

@@ -204,15 +204,22 @@ def self_attn_forward(self, hidden_states: torch.Tensor, kv_cache: Optional[Laye
         lo, hi = st.length, st.length + T
         cos, sin = _rope_table(hi, theta, q.dtype, q.device)
         cos, sin = cos[lo:hi], sin[lo:hi]
-        qr = _rotate(q, cos[None, :, None, :], sin[None, :, None, :])
-        st.k[:, lo:hi] = _rotate(k, cos[None, :, None, :], sin[None, :, None, :])
-        st.v[:, lo:hi] = v
+        native = ops.prefill_covers(q, k, v, st.k, st.v)
+        if native:
+            qr = ops.rope_append(q, k, v, cos, sin, lo, st.k, st.v)
+        else:
+            qr = _rotate(q, cos[None, :, None, :], sin[None, :, None, :])
+            st.k[:, lo:hi] = _rotate(k, cos[None, :, None, :], sin[None, :, None, :])
+            st.v[:, lo:hi] = v
         if hashed:
             if per_q:   # every query head's own code of the shared key (repeat_kv, then hash_fn, spotlight_generation.py:128,17)
                 ops.hash_encode(st.k[:, lo:hi].repeat_interleave(G, dim=2), self._hash_q_params(), out=st.codes[:, lo:hi])
             else:
                 ops.hash_encode(st.k[:, lo:hi], self._hash_k_params(), out=st.codes[:, lo:hi])
         st.length = hi
+        if native:
+            return self.o_proj(ops.prefill_attention(qr, st.k, st.v, lo).view(B, T, num_heads * head_dim)), st
+        # other dtypes, and whatever autograd has to see: torch's attention under the same mask
         kk = st.k[:, :hi].permute(0, 2, 1, 3)
         vv = st.v[:, :hi].permute(0, 2, 1, 3)
         mask = torch.ones((T, hi), dtype=torch.bool, device=q.device).tril(diagonal=hi - T)

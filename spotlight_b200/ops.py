@@ -390,6 +390,70 @@ def hash_encode(x: torch.Tensor, params: HashParams, out: Optional[torch.Tensor]
     return out
 
 
+# ----------------------------------------------------------------------------- a prompt
+def untraced(*tensors: torch.Tensor) -> bool:
+    """Plain tensors nobody differentiates or traces: a kernel may take them behind autograd's back."""
+    if any(type(t) not in (torch.Tensor, torch.nn.Parameter) for t in tensors):
+        return False
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return False
+    return torch.autograd.forward_ad._current_level < 0 and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+
+
+def prefill_covers(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor) -> bool:
+    """Whether rope_append + prefill_attention take these tensors: plain bf16 CUDA tensors nobody differentiates or
+    traces, q [B,T,QH,128] and k / v [B,T,KH,128] with QH a multiple of KH (at most 128 times), cache views whose rows
+    are 16-byte aligned and whose batch rows are distinct."""
+    ts = (q, k, v, k_cache, v_cache)
+    if not untraced(*ts) or any(t.dtype != torch.bfloat16 or not t.is_cuda or t.device != q.device for t in ts):
+        return False
+    B, T, QH, D = q.shape
+    KH = k.shape[2]
+    if D != 128 or k.shape != (B, T, KH, 128) or v.shape != k.shape or QH % KH or QH // KH > 128:
+        return False
+    for c in (k_cache, v_cache):
+        sb, st, sh, sd = c.stride()
+        if sd != 1 or st < 128 or sh < 128 or sb % 8 or st % 8 or sh % 8 or c.data_ptr() % 16 or (B > 1 and sb <= 0):
+            return False
+    return k_cache.stride() == v_cache.stride()
+
+
+def rope_append(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: int,
+                k_cache: torch.Tensor, v_cache: torch.Tensor) -> torch.Tensor:
+    """q [B,T,QH,128], k / v [B,T,KH,128], cos / sin [T,128] (rows of positions pos ..): rotates q and k, writes the K / V
+    rows pos .. pos+T-1 of the caches [B,Nmax,KH,128] (views) and returns the rotated q. One launch, bf16."""
+    B, T, QH, _ = q.shape
+    KH = k.shape[2]
+    _cuda(q, k, v, k_cache, v_cache)
+    assert cos.shape == (T, 128) and sin.shape == (T, 128) and cos.dtype == q.dtype and sin.dtype == q.dtype
+    assert k.shape == (B, T, KH, 128) and v.shape == k.shape and pos + T <= k_cache.shape[1], "kv cache is full"
+    q, k, v, cos, sin = (t.contiguous() for t in (q, k, v, cos, sin))
+    out = torch.empty_like(q)
+    kv, kv2 = _kv_layout(k_cache), _kv_layout(v_cache)
+    assert (kv2.batch_stride, kv2.token_stride, kv2.head_stride) == (kv.batch_stride, kv.token_stride, kv.head_stride)
+    check(lib.sl_rope_append(q.data_ptr(), k.data_ptr(), v.data_ptr(), _dt(q), B, T, QH, KH, cos.data_ptr(), sin.data_ptr(),
+                             out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), C.byref(kv), pos, _stream()))
+    _count()
+    return out
+
+
+def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pos: int) -> torch.Tensor:
+    """Causal attention of the tokens at positions pos .. pos+T-1 (q [B,T,QH,128], rotated) over cache rows
+    0 .. pos+T-1 of [B,>=pos+T,KH,128] views; query head j reads kv head j // (QH // KH). bf16 -> [B,T,QH,128]."""
+    B, T, QH, D = q.shape
+    KH = k_cache.shape[2]
+    assert D == 128 and k_cache.dtype == q.dtype and v_cache.dtype == q.dtype and pos + T <= k_cache.shape[1]
+    _cuda(q, k_cache, v_cache)
+    q = q.contiguous()
+    kv, kv2 = _kv_layout(k_cache), _kv_layout(v_cache)
+    assert (kv2.batch_stride, kv2.token_stride, kv2.head_stride) == (kv.batch_stride, kv.token_stride, kv.head_stride)
+    out = torch.empty_like(q)
+    check(lib.sl_prefill_attn(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), _dt(q), C.byref(kv), B, T, QH, KH, pos,
+                              out.data_ptr(), _stream()))
+    _count()
+    return out
+
+
 # ----------------------------------------------------------------------------- attention
 def sparse_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, idx: torch.Tensor,
                        cnt: torch.Tensor, layout: int = GQA_BLOCKED, out: Optional[torch.Tensor] = None,
