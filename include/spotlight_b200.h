@@ -61,8 +61,8 @@ int sl_set_device(int device);
  *   SL_OPT_ATTN_WARPS   warps per CTA of the bf16 attention kernel: 0 (default) by shape, 4 or 8
  *   SL_OPT_PEER_SPIN_LIMIT  polls (100 ns apart) after which the peer-memory exchanges stop waiting for another
  *                       rank's message and set their status word to 3; default 400000, about a second
- *   SL_OPT_HASH_KERNEL  which kernel sl_hash_encode uses for bf16 rows of a 128 -> 256 -> 128 hash: 0 (default)
- *                       by size, 1 the warp-level tensor-core kernel, 2 the tcgen05 / TMEM kernel for every size
+ *   SL_OPT_HASH_KERNEL  which kernel builds the codes of many bf16 rows: 0 (default) and 2 the tcgen05 / TMEM kernel where it
+ *                       covers the hash, 1 the warp-level tensor-core kernel
  *   SL_OPT_ATTN_CLUSTER 1 (default): the CTAs that share a (batch row, kv head) pair of the bf16 attention kernel form a
  *                       thread-block cluster and combine their partials through distributed shared memory where
  *                       all clusters of the launch fit on the device at once; 0: partials in the workspace and a merge kernel
@@ -231,6 +231,15 @@ int sl_rope_append(const void* d_q, const void* d_k, const void* d_v, int dtype,
  * sl_hash_status. Replaces the dense attention of a prompt (spotlight_generation.py:145-147,217-224). */
 int sl_prefill_attn(const void* d_q, const void* d_k_cache, const void* d_v_cache, int dtype, const sl_kv_layout* kv, int B,
                     int64_t T, int QH, int KH, int64_t pos, void* d_out, void* stream);
+
+/* New rows of one layer, post-RoPE keys and values [B,T,KH,128] (any strides, layouts k_src / v_src), into the caches
+ * (d_k_cache / d_v_cache point at the first new row, geometry kv) and, with a hash, their codes into d_codes [B,T,KH,4]
+ * (first new row, batch stride code_batch_stride words). Rows 16-byte aligned; sources and caches do not overlap. The
+ * tensor-core code builder moves the rows itself; else one copy launch, then sl_hash_encode_ex on the cached rows.
+ * Replaces KVCache.update + KVHash.update of a prompt (spotlight/modifiers/gpu_cache.py:38-45,108-118). */
+int sl_load_rows(const void* d_k, const sl_kv_layout* k_src, const void* d_v, const sl_kv_layout* v_src, int dtype, int B,
+                 int64_t T, int KH, void* d_k_cache, void* d_v_cache, const sl_kv_layout* kv, const sl_hash_params* hash,
+                 uint32_t* d_codes, int64_t code_batch_stride, void* stream);
 
 /* Hash + sign + pack of many rows (code-cache build at prefill):
  * d_x [B,T,H,128] with batch stride x_batch_stride (elements) -> d_codes [B,T,H,4] with batch

@@ -89,6 +89,7 @@ SIGNATURES = {
     "sl_decode_prepare_ex": (_I, [_P, _P, _P, _I, _I, _I, _I, _P, _P, _HP, _HP, _P, _P, _P, _L, _P, _P, _KV, _L, _P]),
     "sl_rope_append": (_I, [_P, _P, _P, _I, _I, _L, _I, _I, _P, _P, _P, _P, _P, _KV, _L, _P]),
     "sl_prefill_attn": (_I, [_P, _P, _P, _I, _KV, _I, _L, _I, _I, _L, _P, _P]),
+    "sl_load_rows": (_I, [_P, _KV, _P, _KV, _I, _I, _L, _I, _P, _P, _KV, _HP, _P, _L, _P]),
     "sl_hash_encode": (_I, [_P, _L, _I, _I, _L, _I, _HP, _P, _L, _P]),
     "sl_hash_encode_ex": (_I, [_P, _L, _L, _L, _I, _I, _L, _I, _HP, _P, _L, _P]),
     "sl_sparse_attn_workspace_bytes": (_Z, [_I, _I, _I]),

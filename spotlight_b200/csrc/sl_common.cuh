@@ -53,6 +53,12 @@ int decode_prepare_impl(const void* d_q, const void* d_k, const void* d_v, int d
                         void* d_k_cache, void* d_v_cache, const sl_kv_layout* kv, int64_t pos, const DevPos* dp,
                         void* stream);
 
+// New rows of a layer's cache: where the K rows that are hashed go, and the V rows beside them (strides in elements).
+struct LoadRows {
+    void* k_cache; void* v_cache; long long cs_b, cs_tok, cs_h;       // at the first new row
+    const void* v; long long vs_b, vs_tok, vs_h;
+};
+
 // ---- launches ----------------------------------------------------------------------------
 // Kernels of the decode path are launched with programmatic stream serialisation: a kernel may
 // start while its predecessor in the stream drains, does whatever does not depend on it, and

@@ -8,26 +8,26 @@
 // accumulators live in tensor memory (TMEM); input tiles arrive by TMA (cp.async.bulk.tensor, one CTA per copy,
 // this GPU's own memory) straight into the same swizzled layout.
 //
-// The MLP kernel (written for a hidden width D1 of 256; 128 halves the pieces). TMEM columns: D1 [0,D1) fp32, H [256,256+D1/2)
-// packed bf16 pairs, D2 [384,512) fp32. Sixteen epilogue warps (a thread owns one row = one TMEM lane and a quarter
-// of the columns) and one issuing thread:
-//   TMA   X tile [128 x 128] into one of two stages            -> x_full[stage]
-//   MMA1  D1[128 x D1] = X W1             (8 x  M128 N=D1 K16)  -> d1_full
+// The MLP kernel keeps TWO tiles in flight, each with 256 columns of TMEM, an input stage, eight epilogue warps and an
+// issuing thread of its own, so that one tile's contractions run under the other's activations (the epilogues take
+// turns). TMEM of a tile: layer 1 in [0,D1); a warp reads the columns 64 w .. (of every 128) of its rows and writes the packed
+// hidden values back over [64 w, +64), columns it has read itself; layer 2's result in [128,256).
+//   TMA   X tile [128 x 128]                                   -> x_full
+//   MMA1  D1[128 x D1] = X W1             (8 x  M128 N=D1 K16)  -> d1_full (the input stage takes the next rows; in the
+//         residual form after h_full, as the epilogue adds the rows)
 //   EPI1  D1 -> registers, torch's rounding points (matmul -> bf16, + bias -> bf16, SiLU -> bf16, + input -> bf16 in the
-//         residual form), packed pairs of bf16 written to H: the A operand of layer 2
-//                                                               -> h_full, h_full2 (a warp's columns in two halves:
-//         MMA2 starts on the first; after the second D1 is free and the input stage takes the next rows; MMA1 of the
-//         next tile, issued behind MMA2 of this one, runs under EPI2)
+//         residual form), packed pairs of bf16 written to H: the A operand of layer 2     -> h_full
 //   MMA2  D2[128 x 128] = H W2            (D1/16 x M128 N128 K16, A from TMEM) -> d2_full
-//   EPI2  D2 -> registers, rounding points, sign bit of every value: a thread holds one 32-bit word of its
-//         row's code and stores it                              -> d2_free
-// SiLU of a bf16 is a function of 16 bits: a table in shared memory, filled by the formula (accurate exp, IEEE division)
-// at the start of the kernel, serves all but exact zeros and outliers, which call the formula; so the codes equal the
-// other kernels' up to the order of the fp32 additions. Still the epilogue takes longer than the contraction: the
-// kernel is bound by instruction issue of the epilogue warps, not by the tensor core. The linear hash has a kernel of
-// its own further down (one contraction per tile, bound by the stream of its input rows). Every wait on an mbarrier is
-// bounded; a wait that runs out raises the library's hash status word, the CTA lets its copies in flight land, frees
-// its TMEM and returns.
+//   EPI2  D2 -> registers, rounding points, sign bit of every value: a thread holds two 32-bit words of its
+//         row's code and stores them                            -> d2_free
+// Bound by the activation: two MUFU operations per hidden value, 4096 clocks per tile of 128 x 256, against 2048 of the tensor
+// core. 128 -> 256 -> 128, 131 072 x 8 rows: 171 us (267 with one tile in flight and a table of SiLU values in
+// shared memory); 128 -> 128 -> 128 residual: 150 us (231). The linear hash has a kernel of its own further
+// down (one contraction per tile, bound by the stream of its input rows). With LOAD the input rows are new rows of a cache: the
+// K rows leave for it from the input stage, the V rows are copied beside them, all by TMA, and the cache is
+// not read back: 131 072 x 8 rows into a fused cache with their codes in 244 us, where two strided copies and the codes took 867.
+// Every wait on an mbarrier is bounded; a wait that runs out raises the library's hash status word, the CTA lets its
+// copies in flight land, frees its TMEM and returns.
 // Same arithmetic as the warp-level kernel in sl_hash_mma.cu up to the order of the fp32 additions.
 #include "sl_common.cuh"
 #include "sl_tc.cuh"
@@ -36,12 +36,20 @@ namespace {
 
 using namespace sltc;
 
-constexpr int TC_EPI_WARPS = 16;                // 4 lane quadrants x 4 column groups
-constexpr int TC_THREADS = (TC_EPI_WARPS + 1) * 32;
+constexpr int TC_EPI_WARPS = 16;                // two tiles x 4 lane quadrants x 2 column halves
+constexpr int TC_THREADS = (TC_EPI_WARPS + 3) * 32;   // + an issuing warp per tile and one that copies V rows
 constexpr int TC_TILE = 128;
-constexpr unsigned W1_BYTES = 128 * 256 * 2, W2_BYTES = 256 * 128 * 2, X_BYTES = TC_TILE * 128 * 2;
-constexpr unsigned OFF_W1 = 0, OFF_W2 = W1_BYTES, OFF_X = W1_BYTES + W2_BYTES, OFF_B1 = OFF_X + 2 * X_BYTES,
-                   OFF_B2 = OFF_B1 + 512, OFF_LUT = OFF_B2 + 256, OFF_BAR = OFF_LUT + 16384, OFF_MISC = OFF_BAR + 8 * 8, TC_SMEM = OFF_MISC + 16 + 1024;
+constexpr unsigned X_BYTES = TC_TILE * 128 * 2, X_SLAB = X_BYTES / 2;
+
+constexpr int VS = 4;                             // pieces of the V copy in flight
+constexpr unsigned V_PIECE = 32 * 256;            // 32 whole rows
+
+// shared memory of the MLP kernel, bytes from a 1024-byte boundary
+template <int D1>
+struct TcSmem {
+    static constexpr unsigned W1 = 0, W2 = 128 * D1 * 2, X = 2 * W2, V = X + 2 * X_BYTES, B1 = V + VS * V_PIECE, B2 = B1 + D1 * 2, BAR = B2 + 256,
+                              MISC = BAR + (12 + VS) * 8, BYTES = MISC + 16 + 1024;
+};
 
 struct HashTcArgs {
     long long T; int H; int B;
@@ -58,19 +66,29 @@ __device__ __forceinline__ unsigned add_bf16x2(unsigned x, unsigned y) {
     return r;
 }
 
-// SiLU of a bf16 at torch's rounding point: fp32 x / (1 + exp(-x)) with the accurate exp and the IEEE division, rounded once.
-__device__ __forceinline__ unsigned short silu_bf16(unsigned short u) {
-    const float y = __uint_as_float((unsigned)u << 16);
-    return __bfloat16_as_ushort(__float2bfloat16_rn(y / (1.0f + expf(-y))));
+// SiLU of a pair of bf16 at torch's rounding point: fp32 x / (1 + exp(-x)), rounded once. Computed as (x/4) * (1 / ((1 + 2^(-x log2 e)) / 4))
+// with the approximate exponential and reciprocal (the quarter keeps the reciprocal of 1 + e^88 out of the denormals,
+// which those flush): over all finite bf16 arguments the rounded result is the one of the accurate formula, bit for bit (tested
+// exhaustively). Two MUFU operations per value; a table of the values in shared memory costs as many clocks (three-way bank
+// conflicts), the index arithmetic and 16 KB that the copy of V rows needs.
+__device__ __forceinline__ unsigned long long pair64(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
 }
-// The activation has one bf16 argument, so it is a function of 16 bits. Its values for 2^-28 <= |x| < 16 (both signs:
-// 8192 arguments, where all of a layer's values lie but exact zeros and outliers) are tabulated in shared memory at the
-// start of the kernel with the formula above; the other arguments go through the formula itself. Either way the
-// result is the formula's, bit for bit.
-constexpr unsigned LUT_LO = 99u << 7;       // 2^-28
-
-__device__ __noinline__ unsigned silu_pair(unsigned y) {
-    return (unsigned)silu_bf16((unsigned short)(y & 0xffffu)) | ((unsigned)silu_bf16((unsigned short)(y >> 16)) << 16);
+__device__ __forceinline__ unsigned silu_pair(unsigned y) {
+    const float NL = -1.4426950408889634f;
+    const unsigned long long x = pair64(__uint_as_float(y << 16), __uint_as_float(y & 0xffff0000u));
+    unsigned long long e, d, r, q;
+    float t0, t1, r0, r1;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(e) : "l"(x), "l"(pair64(NL, NL)));
+    asm("{\n\t.reg .f32 a, b;\n\tmov.b64 {a, b}, %2;\n\tex2.approx.ftz.f32 %0, a;\n\tex2.approx.ftz.f32 %1, b;\n\t}" : "=f"(t0), "=f"(t1) : "l"(e));
+    asm("fma.rn.f32x2 %0, %1, %2, %2;" : "=l"(d) : "l"(pair64(t0, t1)), "l"(pair64(0.25f, 0.25f)));
+    asm("{\n\t.reg .f32 a, b;\n\tmov.b64 {a, b}, %2;\n\trcp.approx.ftz.f32 %0, a;\n\trcp.approx.ftz.f32 %1, b;\n\t}" : "=f"(r0), "=f"(r1) : "l"(d));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(x), "l"(pair64(0.25f, 0.25f)));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(q), "l"(pair64(r0, r1)));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r0), "=f"(r1) : "l"(r));
+    return pack2(r0, r1);
 }
 
 // byte offset of element (row, k) of a K-major operand: slabs of 64 k, rows of 128 bytes, 16-byte chunks XORed with row % 8
@@ -78,44 +96,88 @@ __device__ __forceinline__ unsigned kmajor_off(int row, int k, int rows) {
     return (unsigned)((k >> 6) * rows * 128 + row * 128 + ((((k & 63) >> 3) ^ (row & 7)) << 4) + (k & 7) * 2);
 }
 
-// Phase stamps exist only in profiling builds (-DSL_TC_TIMING): CTA (0,0) stores the SM cycle counter at its phase boundaries.
-#ifdef SL_TC_TIMING
-__device__ unsigned long long g_tc_dbg[2][64][4];
-__device__ unsigned long long g_tc_dbgw[16][4];
-#define TC_STAMPW(k) if (blockIdx.x == 0 && blockIdx.y == 0 && it == 3 && lane == 0) g_tc_dbgw[warp][k] = (unsigned long long)clock64();
-#define TC_STAMP(who, i, k) if (blockIdx.x == 0 && blockIdx.y == 0 && (i) < 64) g_tc_dbg[who][i][k] = (unsigned long long)clock64();
-#else
-#define TC_STAMP(who, i, k)
-#define TC_STAMPW(k)
-#endif
+// LOAD: one thread copies the V rows of the CTA's tiles by TMA, a quarter of a tile (32 whole rows) at a time, VS in
+// flight, one barrier each. False when a bounded wait ran out (its copies have landed all the same).
+__device__ __forceinline__ bool copy_v_rows(unsigned smem, unsigned bars, const CUtensorMap& vsrc, const CUtensorMap& vdst, const HashTcArgs& a,
+                                            long long first, long long step, int h, volatile int* abort_flag) {
+    const long long n = first < a.n_tiles ? 4 * ((a.n_tiles - 1 - first) / step + 1) : 0;
+    auto place = [&](long long i, int& t0, int& b) {
+        const long long tile = first + (i >> 2) * step, bb = tile / a.tiles_per_b;
+        b = (int)bb; t0 = (int)((tile - bb * a.tiles_per_b) * TC_TILE) + (int)(i & 3) * 32;
+    };
+    auto load = [&](long long i) {
+        const unsigned st = (unsigned)(i % VS);
+        int t0, b;
+        place(i, t0, b);
+        mbar_expect_tx(bars + 8u * st, V_PIECE);
+        tma_load_4d(smem + st * V_PIECE, &vsrc, bars + 8u * st, 0, t0, h, b);
+    };
+    long long loaded = 0, i = 0;
+    for (; loaded < VS && loaded < n; ++loaded) load(loaded);
+    bool ok = true;
+    for (; i < n; ++i) {
+        const unsigned st = (unsigned)(i % VS);
+        if (!mbar_wait(bars + 8u * st, (unsigned)(i / VS) & 1u, abort_flag)) { ok = false; break; }
+        int t0, b;
+        place(i, t0, b);
+        if (t0 < a.T) tma_store_4d(&vdst, smem + st * V_PIECE, 0, t0, h, b);
+        bulk_commit();
+        if (i >= 1 && loaded < n) { bulk_wait_read1(); load(loaded); ++loaded; }      // into the piece before this one, which has left
+    }
+    bulk_wait_read();
+    for (; i < loaded; ++i)
+        for (unsigned k = 0; k < WAIT_LIMIT && !mbar_test(bars + 8u * (unsigned)(i % VS), (unsigned)(i / VS) & 1u); ++k) __nanosleep(256);
+    return ok;
+}
 
-// D1: width of the hidden layer (256, or 128: then a warp's columns are one piece and both halves of H arrive together).
-// RES (D1 == 128): the reference's residual form, layer output = f(x W + b) + input, rounded once more to bf16.
-template <int D1, bool RES>
-__global__ void __launch_bounds__(TC_THREADS, 1) hash_encode_tc_kernel(const __grid_constant__ CUtensorMap xmap, const HashTcArgs a) {
+// Sign bits of 16 pairs of bf16 as a code word: bit 2e <- low half > 0, bit 2e + 1 <- high half > 0 of pair e.
+__device__ __forceinline__ unsigned signs16(const unsigned (&y)[16]) {
+    unsigned w[2] = {0u, 0u};                 // eight pairs each: low halves in the even bits 0.., high halves in the even bits 16..
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        __nv_bfloat162 v, z;
+        reinterpret_cast<unsigned&>(v) = y[e];
+        reinterpret_cast<unsigned&>(z) = 0u;
+        w[e >> 3] |= __hgt2_mask(v, z) & (0x00010001u << (2 * (e & 7)));
+    }
+    return (w[0] & 0xffffu) | ((w[0] >> 16) << 1) | (w[1] << 16) | ((w[1] >> 16) << 17);
+}
+
+// D1: width of the hidden layer. RES (D1 == 128): the reference's residual form, layer output = f(x W + b) + input,
+// rounded once more to bf16. LOAD: the input rows are new rows of a cache; the CTA stores every input tile from its
+// stage to the K cache by TMA and copies the V rows of the same tile beside it.
+template <int D1, bool RES, bool LOAD>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+hash_encode_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap kdst,
+                      const __grid_constant__ CUtensorMap vsrc, const __grid_constant__ CUtensorMap vdst, const HashTcArgs a) {
     static_assert(D1 == 256 || (D1 == 128), "hidden width");
     static_assert(!RES || D1 == 128, "a residual layer keeps its width");
-    constexpr int NCH = D1 / 128;                             // 32-column pieces of D1 per epilogue warp
+    using S = TcSmem<D1>;
+    constexpr int NCH = D1 / 64;                              // 32-column pieces of D1 per epilogue warp
     extern __shared__ unsigned char smem_raw[];
     const unsigned raw = (unsigned)__cvta_generic_to_shared(smem_raw);
     const unsigned base = (raw + 1023u) & ~1023u;             // operand slabs start on 1024-byte boundaries
     unsigned char* g = smem_raw + (base - raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int h = blockIdx.y;
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(g + OFF_MISC + 4);
-    unsigned* tmem_slot = reinterpret_cast<unsigned*>(g + OFF_MISC);
-    auto bar = [&](int i) { return base + OFF_BAR + (unsigned)i * 8u; };
-    constexpr int X_FULL = 0 /* and 1 */, D1_FULL = 2, H_FULL = 3 /* first half of every warp's columns */, D2_FULL = 4, D2_FREE = 5, H_FULL2 = 6;
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(g + S::MISC + 4);
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(g + S::MISC);
+    auto bar = [&](int i) { return base + S::BAR + (unsigned)i * 8u; };
+    constexpr int X_FULL = 0, D1_FULL = 2, H_FULL = 4, D2_FULL = 6, D2_FREE = 8 /* each + tile in flight */, TURN = 10, V_FULL = 12 /* .. */;
 
     // ---- set-up: barriers, TMEM, this head's weights (transposed to K-major) and biases
     if (tid == 0) {
         *abort_flag = 0;
-        mbar_init(bar(X_FULL), 1); mbar_init(bar(X_FULL + 1), 1); mbar_init(bar(D1_FULL), 1);
-        mbar_init(bar(H_FULL), TC_EPI_WARPS * 32); mbar_init(bar(H_FULL2), TC_EPI_WARPS * 32); mbar_init(bar(D2_FULL), 1); mbar_init(bar(D2_FREE), TC_EPI_WARPS * 32);
+        for (int p = 0; p < 2; ++p) {
+            mbar_init(bar(X_FULL + p), 1); mbar_init(bar(D1_FULL + p), 1); mbar_init(bar(D2_FULL + p), 1);
+            mbar_init(bar(H_FULL + p), TC_EPI_WARPS * 16); mbar_init(bar(D2_FREE + p), TC_EPI_WARPS * 16);
+            mbar_init(bar(TURN + p), TC_EPI_WARPS * 16);
+        }
+        for (int i = 0; i < VS; ++i) mbar_init(bar(V_FULL + i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == TC_EPI_WARPS) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(base + OFF_MISC) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(base + S::MISC) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     {
@@ -129,7 +191,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) hash_encode_tc_kernel(const __g
             const uint4 v = w1[k * NG1 + (task % NG1)];
             const unsigned short* e = reinterpret_cast<const unsigned short*>(&v);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) *reinterpret_cast<unsigned short*>(g + OFF_W1 + kmajor_off(n0 + c, k, D1)) = e[c];
+            for (int c = 0; c < 8; ++c) *reinterpret_cast<unsigned short*>(g + S::W1 + kmajor_off(n0 + c, k, D1)) = e[c];
         }
         const uint4* w2 = reinterpret_cast<const uint4*>(a.w2 + (long long)h * D1 * 128);         // [k][n], 16 groups of 8 n per row
         for (int task = warp; task < (D1 / 32) * 16; task += NWARP) {
@@ -137,15 +199,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) hash_encode_tc_kernel(const __g
             const uint4 v = w2[k * 16 + (task & 15)];
             const unsigned short* e = reinterpret_cast<const unsigned short*>(&v);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) *reinterpret_cast<unsigned short*>(g + OFF_W2 + kmajor_off(n0 + c, k, 128)) = e[c];
+            for (int c = 0; c < 8; ++c) *reinterpret_cast<unsigned short*>(g + S::W2 + kmajor_off(n0 + c, k, 128)) = e[c];
         }
-        __nv_bfloat16* sb1 = reinterpret_cast<__nv_bfloat16*>(g + OFF_B1);
-        __nv_bfloat16* sb2 = reinterpret_cast<__nv_bfloat16*>(g + OFF_B2);
+        __nv_bfloat16* sb1 = reinterpret_cast<__nv_bfloat16*>(g + S::B1);
+        __nv_bfloat16* sb2 = reinterpret_cast<__nv_bfloat16*>(g + S::B2);
         for (int i = tid; i < D1; i += TC_THREADS) sb1[i] = a.b1 ? a.b1[(long long)h * D1 + i] : __float2bfloat16_rn(0.0f);
         for (int i = tid; i < 128; i += TC_THREADS) sb2[i] = a.b2 ? a.b2[(long long)h * 128 + i] : __float2bfloat16_rn(0.0f);
-        unsigned short* lut = reinterpret_cast<unsigned short*>(g + OFF_LUT);
-        for (unsigned i = tid; i < 8192u; i += TC_THREADS)
-            lut[i] = silu_bf16((unsigned short)(((i & 0xfffu) + LUT_LO) | ((i & 0x1000u) << 3)));
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the weights were written by ordinary stores, the tensor core reads them
     tc_fence_before();
@@ -153,159 +212,141 @@ __global__ void __launch_bounds__(TC_THREADS, 1) hash_encode_tc_kernel(const __g
     tc_fence_after();
     const unsigned tmem = *tmem_slot;
 
-    const long long first = blockIdx.x, step = gridDim.x;
+    const long long first = blockIdx.x, step = gridDim.x;            // this CTA's tiles; tile in flight p takes every second one
     bool failed = false;
 
     if (warp < TC_EPI_WARPS) {
-        // ================= epilogue warps: thread = row = TMEM lane, warp group cg = a quarter of the columns =================
-        const int q = warp & 3, cg = warp >> 2, row = q * 32 + lane;
-        const unsigned t_row = tmem + ((unsigned)(q * 32) << 16);
-        const unsigned t_d1 = t_row + (unsigned)(D1 / 4) * cg, t_h = t_row + 256u + (unsigned)(D1 / 8) * cg, t_d2 = t_row + 384u + 32u * cg;
-        const unsigned* sb1 = reinterpret_cast<const unsigned*>(g + OFF_B1) + (D1 / 8) * cg;     // pairs of bf16
-        unsigned hk[16];                                       // RES: this thread's 32 hidden values, the residual of layer 2
-        const unsigned* sb2 = reinterpret_cast<const unsigned*>(g + OFF_B2) + 16 * cg;
-        const unsigned char* lutb = g + OFF_LUT;
+        // ================= epilogue warps: thread = row = TMEM lane and a half of the columns of tile in flight p =================
+        const int p = warp >> 3, q = warp & 3, hw = (warp >> 2) & 1, row = q * 32 + lane;
+        const unsigned t_row = tmem + ((unsigned)(q * 32) << 16) + 256u * p;
+        const unsigned t_d1 = t_row + 64u * hw, t_d2 = t_row + 128u + 64u * hw;
+        const unsigned* sb1 = reinterpret_cast<const unsigned*>(g + S::B1) + 32 * hw;           // pairs of bf16
+        auto piece = [](int jj) { return 32 * jj + (jj >= 2 ? 64 : 0); };                       // its jj-th 32 columns, from 64 hw
+        const unsigned* sb2 = reinterpret_cast<const unsigned*>(g + S::B2) + 32 * hw;
+        unsigned hk[RES ? 32 : 1];                             // RES: this thread's 64 hidden values, the residual of layer 2
+        const unsigned char* xrow = g + S::X + p * X_BYTES + hw * X_SLAB;           // RES: a column half is a slab of the input stage
         unsigned it = 0;
-        for (long long tile = first; tile < a.n_tiles; tile += step, ++it) {
+        for (long long tile = first + p * step; tile < a.n_tiles; tile += 2 * step, ++it) {
             const unsigned par = it & 1u;
-            if (!__all_sync(0xffffffffu, mbar_wait(bar(D1_FULL), par, abort_flag))) { failed = true; break; }   // warp-uniform: the TMEM accesses below are warp-wide
+            if (!__all_sync(0xffffffffu, mbar_wait(bar(D1_FULL + p), par, abort_flag))) { failed = true; break; }   // warp-uniform: the TMEM accesses below are warp-wide
             tc_fence_after();
-            if (tid == 0) { TC_STAMP(0, it, 0) }
-            TC_STAMPW(0)
-            unsigned v[1][32];
-#pragma unroll 1
+            // its turn: one tile's activations at a time. Both epilogues want the same unit (MUFU); let run side by side they fall into
+            // step and leave it idle while both wait for their contractions
+            if ((it > 0 || p == 1) && !__all_sync(0xffffffffu, mbar_wait(bar(TURN + p), p == 1 ? par : par ^ 1u, abort_flag))) { failed = true; break; }
+            unsigned raw1[2][32];
+            tmem_ld32(t_d1, raw1[0]);
+#pragma unroll
             for (int jj = 0; jj < NCH; ++jj) {
-                constexpr int j = 0;
-                unsigned pk[16], oob = 0u;
-                tmem_ld32(t_d1 + 32u * jj, v[0]);
+                unsigned (&v)[32] = raw1[jj & 1];
+                unsigned pk[16];
                 tmem_wait_ld();
+                if (jj == NCH - 1) mbar_arrive(bar(TURN + (p ^ 1)));                                     // the other tile starts under the last piece
+                if (jj + 1 < NCH) tmem_ld32(t_d1 + piece(jj + 1), raw1[(jj + 1) & 1]);                  // on its way under this piece's work
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
-                    unsigned y = pack2(__uint_as_float(v[j][2 * e]), __uint_as_float(v[j][2 * e + 1]));   // matmul -> bf16
-                    y = add_bf16x2(y, sb1[16 * jj + e]);                                                   // + bias -> bf16 (a null bias is a row of zeros)
-                    v[j][e] = y;
-                    // both halves at once: a half outside the table's range leaves bits in 0x7000 (a borrow from the low half can
-                    // only come from such a half), and then the pair goes through the formula below
-                    const unsigned d = y - (LUT_LO | (LUT_LO << 16)), dh = d >> 16;
-                    oob |= d;
-                    const unsigned i0 = ((d << 1) & 0x1ffeu) | ((d >> 2) & 0x2000u), i1 = ((dh << 1) & 0x1ffeu) | ((dh >> 2) & 0x2000u);
-                    pk[e] = (unsigned)*reinterpret_cast<const unsigned short*>(lutb + i0) |
-                            ((unsigned)*reinterpret_cast<const unsigned short*>(lutb + i1) << 16);         // SiLU -> bf16
-                }
-                if (oob & 0x70007000u) {
-#pragma unroll
-                    for (int e = 0; e < 16; ++e)                                  // only the pairs that need it (an exact zero, mostly: a sum that
-                        if ((v[j][e] - (LUT_LO | (LUT_LO << 16))) & 0x70007000u)  // cancelled its bias); a call each, so the arrays stay in registers
-                            pk[e] = silu_pair(v[j][e]);
+                    unsigned y = pack2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));         // matmul -> bf16
+                    y = add_bf16x2(y, sb1[piece(jj) / 2 + e]);                                                   // + bias -> bf16 (a null bias is a row of zeros)
+                    pk[e] = silu_pair(y);                                                                  // SiLU -> bf16
                 }
                 if (RES) {                  // + input -> bf16: the thread's own row of the tile, still in its input stage
-                    const unsigned char* xrow = g + OFF_X + (it & 1u) * X_BYTES;
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
-                        pk[e] = add_bf16x2(pk[e], *reinterpret_cast<const unsigned*>(xrow + kmajor_off(row, 32 * cg + 2 * e, TC_TILE)));
-                        hk[e] = pk[e];
+                        pk[e] = add_bf16x2(pk[e], *reinterpret_cast<const unsigned*>(xrow + kmajor_off(row, 32 * jj + 2 * e, TC_TILE)));
+                        hk[(16 * jj + e) & (RES ? 31 : 0)] = pk[e];
                     }
                 }
-                tmem_st16(t_h + 16u * jj, pk);
-                tmem_wait_st();
-                tc_fence_before();
-                if (NCH == 1 || jj == 0) mbar_arrive(bar(H_FULL));     // layer 2 starts on the half that is there
-                if (NCH == 1 || jj == 1) mbar_arrive(bar(H_FULL2));
+                tmem_st16(t_d1 + 16u * jj, pk);               // over columns this warp has read
             }
-            if (tid == 0) { TC_STAMP(0, it, 1) }
-            TC_STAMPW(1)
+            tmem_wait_st();
+            tc_fence_before();
+            mbar_arrive(bar(H_FULL + p));
 
-            if (!__all_sync(0xffffffffu, mbar_wait(bar(D2_FULL), par, abort_flag))) { failed = true; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(bar(D2_FULL + p), par, abort_flag))) { failed = true; break; }
             tc_fence_after();
-            if (tid == 0) { TC_STAMP(0, it, 2) }
-            TC_STAMPW(2)
+            unsigned v[2][32];
             tmem_ld32(t_d2, v[0]);
+            tmem_ld32(t_d2 + 32u, v[1]);
             tmem_wait_ld();
             tc_fence_before();
-            mbar_arrive(bar(D2_FREE));
-            unsigned bits = 0u;
+            mbar_arrive(bar(D2_FREE + p));
+            unsigned word[2];
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                unsigned y = pack2(__uint_as_float(v[0][2 * e]), __uint_as_float(v[0][2 * e + 1]));
-                y = add_bf16x2(y, sb2[e]);
-                if (RES) y = add_bf16x2(y, hk[e]);              // + the layer's input (the hidden values of the same columns)
-                const float y0 = __uint_as_float(y << 16), y1 = __uint_as_float(y & 0xffff0000u);
-                bits |= ((y0 > 0.0f ? 1u : 0u) | (y1 > 0.0f ? 2u : 0u)) << (2 * e);
+            for (int j = 0; j < 2; ++j) {
+                unsigned y[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    y[e] = add_bf16x2(pack2(__uint_as_float(v[j][2 * e]), __uint_as_float(v[j][2 * e + 1])), sb2[16 * j + e]);
+                    if (RES) y[e] = add_bf16x2(y[e], hk[(16 * j + e) & (RES ? 31 : 0)]);   // + the layer's input (the hidden values of the same columns)
+                }
+                word[j] = signs16(y);
             }
             const long long b = tile / a.tiles_per_b, t = (tile - b * a.tiles_per_b) * TC_TILE + row;
-            if (t < a.T) a.codes[b * a.cs_b + (t * a.H + h) * 4 + cg] = bits;
-            if (tid == 0) { TC_STAMP(0, it, 3) }
-            TC_STAMPW(3)
+            if (t < a.T) *reinterpret_cast<uint2*>(a.codes + b * a.cs_b + (t * a.H + h) * 4 + 2 * hw) = make_uint2(word[0], word[1]);
         }
-    } else if (lane == 0) {
-        // ================= issuing thread: TMA loads and tensor-core instructions =================
-        const unsigned x_s = base + OFF_X;
+    } else if (warp < TC_EPI_WARPS + 2 && lane == 0) {
+        // ================= issuing thread of tile in flight p: TMA copies and tensor-core instructions =================
+        const int p = warp - TC_EPI_WARPS;
+        const unsigned x_s[2] = {base + S::X + p * X_BYTES, base + S::X + p * X_BYTES + X_SLAB}, tm = tmem + 256u * p;
         constexpr unsigned I1 = instr_desc(D1), I2 = instr_desc(128);
-        bool pending[2] = {false, false};                     // a copy into this stage is in flight
-        auto load = [&](long long tile, int st) {
-            const long long b = tile / a.tiles_per_b;
-            const int t0 = (int)((tile - b * a.tiles_per_b) * TC_TILE);
-            const unsigned dst = x_s + (unsigned)st * X_BYTES;
-            mbar_expect_tx(bar(X_FULL + st), X_BYTES);
-            tma_load_4d(dst, &xmap, bar(X_FULL + st), 0, t0, h, (int)b);                 // k 0..63 of the 128 rows
-            tma_load_4d(dst + X_BYTES / 2, &xmap, bar(X_FULL + st), 64, t0, h, (int)b);  // k 64..127
-            pending[st] = true;
+        unsigned loads = 0;
+        auto coords = [&](long long tile, int& t0, int& b) {
+            const long long bb = tile / a.tiles_per_b;
+            b = (int)bb;
+            t0 = (int)((tile - bb * a.tiles_per_b) * TC_TILE);
         };
-        auto mma1 = [&](unsigned n) -> bool {                 // layer 1 of this CTA's n-th tile, once its rows have landed
-            const int st = (int)(n & 1u);
-            if (!mbar_wait(bar(X_FULL + st), (n >> 1) & 1u, abort_flag)) return false;
-            pending[st] = false;
+        auto load = [&](long long tile) {
+            int t0, b;
+            coords(tile, t0, b);
+            if (LOAD) bulk_wait_read();                       // the stage's rows have left for the cache
+            mbar_expect_tx(bar(X_FULL + p), X_BYTES);
+            tma_load_4d(x_s[0], &xmap, bar(X_FULL + p), 0, t0, h, b);              // k 0..63 of the 128 rows
+            tma_load_4d(x_s[1], &xmap, bar(X_FULL + p), 64, t0, h, b);             // k 64..127
+            ++loads;
+        };
+        long long tile = first + p * step;
+        if (tile < a.n_tiles) load(tile);
+        unsigned it = 0;
+        for (; tile < a.n_tiles; tile += 2 * step, ++it) {
+            const unsigned par = it & 1u;
+            if (!mbar_wait(bar(X_FULL + p), par, abort_flag)) { failed = true; break; }
+            if (it > 0 && !mbar_wait(bar(D2_FREE + p), par ^ 1u, abort_flag)) { failed = true; break; }   // the tile before is out of TMEM
             tc_fence_after();
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks) {
-                const unsigned ao = (unsigned)st * X_BYTES + (unsigned)(ks >> 2) * (X_BYTES / 2) + (unsigned)(ks & 3) * 32u;
                 const unsigned bo = (unsigned)(ks >> 2) * ((unsigned)D1 * 128u) + (unsigned)(ks & 3) * 32u;
-                mma_ss(tmem, smem_desc(x_s + ao), smem_desc(base + OFF_W1 + bo), I1, ks > 0 ? 1u : 0u);
+                mma_ss(tm, smem_desc(x_s[ks >> 2] + (unsigned)(ks & 3) * 32u), smem_desc(base + S::W1 + bo), I1, ks > 0 ? 1u : 0u);
             }
-            tc_commit(bar(D1_FULL));
-            return true;
-        };
-        if (first < a.n_tiles) load(first, 0);
-        if (first + step < a.n_tiles) load(first + step, 1);
-        if (first < a.n_tiles && !mma1(0)) failed = true;
-        unsigned it = 0;
-        for (long long tile = first; tile < a.n_tiles && !failed; tile += step, ++it) {
-            const unsigned par = it & 1u;
-            TC_STAMP(1, it, 0)
-            if (!mbar_wait(bar(H_FULL), par, abort_flag)) { failed = true; break; }        // the first half of every warp's H columns is written
-            TC_STAMP(1, it, 1)
-            if (it > 0 && !mbar_wait(bar(D2_FREE), par ^ 1u, abort_flag)) { failed = true; break; }   // D2 of the previous tile has been read
+            tc_commit(bar(D1_FULL + p));
+            if (LOAD) {
+                int t0, b;
+                coords(tile, t0, b);
+                tma_store_4d(&kdst, x_s[0], 0, t0, h, b);
+                tma_store_4d(&kdst, x_s[1], 64, t0, h, b);
+                bulk_commit();
+            }
+            if (!RES) {                                       // layer 1 is over: the stage takes the next rows
+                if (!mbar_wait(bar(D1_FULL + p), par, abort_flag)) { failed = true; break; }
+                if (tile + 2 * step < a.n_tiles) load(tile + 2 * step);
+            }
+            if (!mbar_wait(bar(H_FULL + p), par, abort_flag)) { failed = true; break; }
             tc_fence_after();
+            if (RES && tile + 2 * step < a.n_tiles) load(tile + 2 * step);         // the input rows have been added
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                if (half == 1) {
-                    if (!mbar_wait(bar(H_FULL2), par, abort_flag)) { failed = true; break; }   // the rest of H is written, all of D1 read
-                    tc_fence_after();
-                    // layer 1 of this tile is over and (RES) its input rows have been added: the input stage takes the next rows
-                    if (tile + 2 * step < a.n_tiles) load(tile + 2 * step, (int)par);
-                }
-                if (NCH == 2 || half == 0) {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        // D1 = 256: warp group cg wrote K [64 cg + 32 half, + 32); D1 = 128: K [32 cg, + 32), all there at once
-                        const int ks = NCH == 2 ? 4 * (i >> 1) + 2 * half + (i & 1) : i;
-                        const unsigned bo = (unsigned)(ks >> 2) * (128u * 128u) + (unsigned)(ks & 3) * 32u;
-                        mma_ts(tmem + 384u, tmem + 256u + 8u * ks, smem_desc(base + OFF_W2 + bo), I2, (half | i) ? 1u : 0u);
-                    }
-                }
+            for (int i = 0; i < D1 / 16; ++i) {
+                // D1 = 256: the order of the sums stays the one of the kernel before this one (0 1 4 5 8 9 12 13, then 2 3 6 7 ..): codes
+                // built by either are the same bit for bit
+                const int ks = D1 == 256 ? 4 * ((i & 7) >> 1) + 2 * (i >> 3) + (i & 1) : i;
+                const unsigned ho = (unsigned)((ks >> 2) & 1) * 64u + (unsigned)(ks >> 3) * 32u + (unsigned)(ks & 3) * 8u;
+                const unsigned bo = (unsigned)(ks >> 2) * (128u * 128u) + (unsigned)(ks & 3) * 32u;
+                mma_ts(tm + 128u, tm + ho, smem_desc(base + S::W2 + bo), I2, i > 0 ? 1u : 0u);
             }
-            if (failed) break;
-            tc_commit(bar(D2_FULL));
-            TC_STAMP(1, it, 2)
-            if (tile + step < a.n_tiles && !mma1(it + 1)) { failed = true; break; }         // runs under the second epilogue of this tile
+            tc_commit(bar(D2_FULL + p));
         }
-        TC_STAMP(1, 63, 3)
-        if (failed) {                                         // copies of ours still in flight: let them land (bounded)
-            for (int st = 0; st < 2; ++st)
-                if (pending[st]) {
-                    for (unsigned i = 0; i < WAIT_LIMIT && !(mbar_test(bar(X_FULL + st), 0u) || mbar_test(bar(X_FULL + st), 1u)); ++i) __nanosleep(256);
-                }
-        }
+        if (LOAD) bulk_wait_read();
+        if (failed && loads > 0)                              // a copy of ours may still be in flight: let it land (bounded)
+            for (unsigned i = 0; i < WAIT_LIMIT && !mbar_test(bar(X_FULL + p), (loads - 1u) & 1u); ++i) __nanosleep(256);
+    } else if (LOAD && warp == TC_EPI_WARPS + 2 && lane == 0) {
+        failed = !copy_v_rows(base + S::V, bar(V_FULL), vsrc, vdst, a, first, step, h, abort_flag);
     }
     if (failed) {
         *abort_flag = 1;
@@ -322,11 +363,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) hash_encode_tc_kernel(const __g
 // keeps four input stages in flight and two accumulators in TMEM; two teams of four epilogue warps take alternate
 // tiles (a thread reads its row's 128 columns, adds the bias, takes the sign bits and stores the row's 16-byte code).
 constexpr int L1_NS = 4;                        // input stages
-constexpr int L1_THREADS = (8 + 1) * 32;
-constexpr unsigned L1_W = 128 * 128 * 2, L1_OFF_X = L1_W, L1_OFF_B = L1_OFF_X + L1_NS * X_BYTES, L1_OFF_BAR = L1_OFF_B + 256,
-                   L1_OFF_MISC = L1_OFF_BAR + 8 * 8, L1_SMEM = L1_OFF_MISC + 16 + 1024;
+constexpr int L1_THREADS = (8 + 2) * 32;
+constexpr unsigned L1_W = 128 * 128 * 2, L1_OFF_X = L1_W, L1_OFF_V = L1_OFF_X + L1_NS * X_BYTES, L1_OFF_B = L1_OFF_V + VS * V_PIECE,
+                   L1_OFF_BAR = L1_OFF_B + 256, L1_OFF_MISC = L1_OFF_BAR + (8 + VS) * 8, L1_SMEM = L1_OFF_MISC + 16 + 1024;
 
-__global__ void __launch_bounds__(L1_THREADS, 1) hash_encode_tc_linear_kernel(const __grid_constant__ CUtensorMap xmap, const HashTcArgs a) {
+template <bool LOAD>
+__global__ void __launch_bounds__(L1_THREADS, 1)
+hash_encode_tc_linear_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap kdst,
+                             const __grid_constant__ CUtensorMap vsrc, const __grid_constant__ CUtensorMap vdst, const HashTcArgs a) {
     extern __shared__ unsigned char smem_raw[];
     const unsigned raw = (unsigned)__cvta_generic_to_shared(smem_raw);
     const unsigned base = (raw + 1023u) & ~1023u;
@@ -336,11 +380,12 @@ __global__ void __launch_bounds__(L1_THREADS, 1) hash_encode_tc_linear_kernel(co
     volatile int* abort_flag = reinterpret_cast<volatile int*>(g + L1_OFF_MISC + 4);
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(g + L1_OFF_MISC);
     auto bar = [&](int i) { return base + L1_OFF_BAR + (unsigned)i * 8u; };
-    constexpr int X_FULL = 0 /* .. 3 */, D_FULL = 4 /* , 5 */, D_FREE = 6 /* , 7 */;
+    constexpr int X_FULL = 0 /* .. 3 */, D_FULL = 4 /* , 5 */, D_FREE = 6 /* , 7 */, V_FULL = 8 /* .. */;
 
     if (tid == 0) {
         *abort_flag = 0;
         for (int i = 0; i < L1_NS; ++i) mbar_init(bar(X_FULL + i), 1);
+        for (int i = 0; i < VS; ++i) mbar_init(bar(V_FULL + i), 1);
         for (int i = 0; i < 2; ++i) { mbar_init(bar(D_FULL + i), 1); mbar_init(bar(D_FREE + i), 128); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -386,20 +431,16 @@ __global__ void __launch_bounds__(L1_THREADS, 1) hash_encode_tc_linear_kernel(co
             unsigned word[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                unsigned bits = 0u;
+                unsigned y[16];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    unsigned y = pack2(__uint_as_float(v[j][2 * e]), __uint_as_float(v[j][2 * e + 1]));   // matmul -> bf16
-                    y = add_bf16x2(y, sb[16 * j + e]);                                                     // + bias -> bf16
-                    const float y0 = __uint_as_float(y << 16), y1 = __uint_as_float(y & 0xffff0000u);
-                    bits |= ((y0 > 0.0f ? 1u : 0u) | (y1 > 0.0f ? 2u : 0u)) << (2 * e);
-                }
-                word[j] = bits;
+                for (int e = 0; e < 16; ++e)                                                               // matmul -> bf16, + bias -> bf16
+                    y[e] = add_bf16x2(pack2(__uint_as_float(v[j][2 * e]), __uint_as_float(v[j][2 * e + 1])), sb[16 * j + e]);
+                word[j] = signs16(y);
             }
             const long long b = tile / a.tiles_per_b, t = (tile - b * a.tiles_per_b) * TC_TILE + row;
             if (t < a.T) *reinterpret_cast<uint4*>(a.codes + b * a.cs_b + (t * a.H + h) * 4) = make_uint4(word[0], word[1], word[2], word[3]);
         }
-    } else if (lane == 0) {
+    } else if (warp == 8 && lane == 0) {
         // ================= issuing thread =================
         const unsigned x_s = base + L1_OFF_X;
         constexpr unsigned I1 = instr_desc(128);
@@ -429,18 +470,29 @@ __global__ void __launch_bounds__(L1_THREADS, 1) hash_encode_tc_linear_kernel(co
                 mma_ss(tmem + 128u * buf, smem_desc(x_s + ao), smem_desc(base + bo), I1, ks > 0 ? 1u : 0u);
             }
             tc_commit(bar(D_FULL + buf));
+            if (LOAD) {
+                const long long b = tile / a.tiles_per_b;
+                const int t0 = (int)((tile - b * a.tiles_per_b) * TC_TILE);
+                tma_store_4d(&kdst, x_s + (unsigned)st * X_BYTES, 0, t0, h, (int)b);
+                tma_store_4d(&kdst, x_s + (unsigned)st * X_BYTES + X_SLAB, 64, t0, h, (int)b);
+                bulk_commit();
+            }
             if (it >= 1) {       // the contraction of the tile before this one is over by now or soon: its input stage takes the next rows
                 if (!mbar_wait(bar(D_FULL + (buf ^ 1)), ((it - 1u) >> 1) & 1u, abort_flag)) { failed = true; break; }
                 const long long nxt = tile + (long long)(L1_NS - 1) * step;
+                if (LOAD) bulk_wait_read1();                  // that tile's rows have left for the cache (this one's may still be leaving)
                 if (nxt < a.n_tiles) load(nxt, (int)((it - 1u) % L1_NS));
             }
         }
+        if (LOAD) bulk_wait_read();
         if (failed) {
             for (int st = 0; st < L1_NS; ++st)
                 if (pending[st]) {
                     for (unsigned i = 0; i < WAIT_LIMIT && !(mbar_test(bar(X_FULL + st), 0u) || mbar_test(bar(X_FULL + st), 1u)); ++i) __nanosleep(256);
                 }
         }
+    } else if (LOAD && warp == 9 && lane == 0) {
+        failed = !copy_v_rows(base + L1_OFF_V, bar(V_FULL), vsrc, vdst, a, first, step, h, abort_flag);
     }
     if (failed) {
         *abort_flag = 1;
@@ -454,16 +506,9 @@ __global__ void __launch_bounds__(L1_THREADS, 1) hash_encode_tc_linear_kernel(co
 }
 
 int* g_status_host = nullptr;     // one mapped host word for the process: any device and any of the tensor-core kernels may raise it
-int g_hash_kernel = 0;            // 0 by shape, 1 warp-level kernel only, 2 this kernel whenever it covers the shape
+int g_hash_kernel = 0;            // 1: warp-level kernel only; else this kernel whenever it covers the shape
 
 }  // namespace
-
-#ifdef SL_TC_TIMING
-extern "C" int sl_profile_tc_timing(unsigned long long* host_out) {
-    if (cudaMemcpyFromSymbol(host_out + 2 * 64 * 4, g_tc_dbgw, sizeof(g_tc_dbgw)) != cudaSuccess) return 1;
-    return cudaMemcpyFromSymbol(host_out, g_tc_dbg, sizeof(g_tc_dbg)) == cudaSuccess ? 0 : 1;
-}
-#endif
 
 namespace sl {
 
@@ -491,28 +536,38 @@ int take_hash_status() {
 }
 
 // Returns SL_OK after launching, 1 when the shape is not one this kernel covers (the caller falls through to the
-// warp-level kernel), or an error code.
+// warp-level kernel), or an error code. With `load` the rows are also stored to the K cache and their V rows copied.
 int launch_hash_encode_tc(const void* x, long long xs_b, long long xs_tok, long long xs_h, int B, long long T, int H, const sl_hash_params* hp,
-                          uint32_t* codes, long long cs_b, cudaStream_t s) {
+                          uint32_t* codes, long long cs_b, const LoadRows* load, cudaStream_t s) {
     if (g_hash_kernel == 1) return 1;
     const bool mlp = hp->n_layers == 2 && hp->dims[0] == 128 && (hp->dims[1] == 256 || hp->dims[1] == 128) && hp->dims[2] == 128;
     const bool linear = hp->n_layers == 1 && hp->dims[0] == 128 && hp->dims[1] == 128;
     if ((!mlp && !linear) || (hp->residue && (linear || hp->dims[1] != 128))) return 1;
     if (H > 65535 || B > 65535 || T > 0x7fffff00ll) return 1;
-    if (g_hash_kernel == 0 && (long long)B * T * H < 32768) return 1;           // too few tiles to pay for the set-up
+    // no lower limit on the rows: from 64 rows up this kernel takes as long as the warp-level one or less (1024 rows of 8 heads: 18.5 us
+    // against 32.9 with a hidden layer of 256, 12.7 against 20.9 with 128, equal for the linear hash)
     if (!sl::aligned16(x) || !sl::aligned16(codes) || cs_b % 4 != 0) return 1;
-    if (xs_tok % 8 != 0 || xs_h % 8 != 0 || (B > 1 && (xs_b % 8 != 0 || xs_b <= 0))) return 1;
     EncodeTiledFn enc = encode_fn();
     if (!enc) return 1;
     int* d_status = sl::tc_status_word();
     if (!d_status) return 1;
 
-    CUtensorMap map;
-    const cuuint64_t gdim[4] = {128, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
-    const cuuint64_t gstr[3] = {(cuuint64_t)xs_tok * 2, (cuuint64_t)xs_h * 2, (cuuint64_t)(B > 1 ? xs_b : (long long)T * xs_tok) * 2};
-    const cuuint32_t box[4] = {64, TC_TILE, 1, 1}, estr[4] = {1, 1, 1, 1};
-    if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    // a map over [B,T,H,128] rows, boxes of 128 rows x 64 columns in the operands' swizzled layout, or (V) of 32 whole rows as they
+    // are; false where TMA cannot address them
+    auto encode = [&](CUtensorMap* map, const void* p, long long st_b, long long st_tok, long long st_h, bool operand = true) {
+        if (!sl::aligned16(p) || st_tok % 8 != 0 || st_h % 8 != 0 || st_tok < 128 || st_h < 128 || (B > 1 && (st_b % 8 != 0 || st_b <= 0))) return false;
+        const cuuint64_t gdim[4] = {128, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
+        const cuuint64_t gstr[3] = {(cuuint64_t)st_tok * 2, (cuuint64_t)st_h * 2, (cuuint64_t)(B > 1 ? st_b : T * st_tok) * 2};
+        const cuuint32_t box[4] = {operand ? 64u : 128u, operand ? (unsigned)TC_TILE : 32u, 1, 1}, estr[4] = {1, 1, 1, 1};
+        return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(p), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   operand ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    CUtensorMap map, kdst, vsrc, vdst;
+    if (!encode(&map, x, xs_b, xs_tok, xs_h)) return 1;
+    kdst = vsrc = vdst = map;
+    if (load && (!encode(&kdst, load->k_cache, load->cs_b, load->cs_tok, load->cs_h) ||
+                 !encode(&vsrc, load->v, load->vs_b, load->vs_tok, load->vs_h, false) ||
+                 !encode(&vdst, load->v_cache, load->cs_b, load->cs_tok, load->cs_h, false)))
         return 1;
 
     HashTcArgs a = {};
@@ -525,16 +580,22 @@ int launch_hash_encode_tc(const void* x, long long xs_b, long long xs_tok, long 
     a.status = d_status;
     const long long per_head = std::max<long long>(1, (long long)sl::sm_count() / H);
     const unsigned gx = (unsigned)std::min<long long>(a.n_tiles, per_head);
-    if (mlp) {
-        void (*kern)(const CUtensorMap, const HashTcArgs) = hp->dims[1] == 256 ? hash_encode_tc_kernel<256, false>
-                                                          : hp->residue       ? hash_encode_tc_kernel<128, true>
-                                                                              : hash_encode_tc_kernel<128, false>;
-        SL_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
-        kern<<<dim3(gx, (unsigned)H), TC_THREADS, TC_SMEM, s>>>(map, a);
+    typedef void (*Kern)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const HashTcArgs);
+    Kern kern;
+    unsigned smem, threads = TC_THREADS;
+    if (!mlp) {
+        kern = load ? (Kern)hash_encode_tc_linear_kernel<true> : (Kern)hash_encode_tc_linear_kernel<false>;
+        smem = L1_SMEM; threads = L1_THREADS;
+    } else if (hp->dims[1] == 256) {
+        kern = load ? (Kern)hash_encode_tc_kernel<256, false, true> : (Kern)hash_encode_tc_kernel<256, false, false>;
+        smem = TcSmem<256>::BYTES;
     } else {
-        SL_CUDA_OK(cudaFuncSetAttribute(hash_encode_tc_linear_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L1_SMEM));
-        hash_encode_tc_linear_kernel<<<dim3(gx, (unsigned)H), L1_THREADS, L1_SMEM, s>>>(map, a);
+        if (hp->residue) kern = load ? (Kern)hash_encode_tc_kernel<128, true, true> : (Kern)hash_encode_tc_kernel<128, true, false>;
+        else kern = load ? (Kern)hash_encode_tc_kernel<128, false, true> : (Kern)hash_encode_tc_kernel<128, false, false>;
+        smem = TcSmem<128>::BYTES;
     }
+    SL_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<dim3(gx, (unsigned)H), threads, smem, s>>>(map, kdst, vsrc, vdst, a);
     SL_CUDA_OK(cudaGetLastError());
     return SL_OK;
 }

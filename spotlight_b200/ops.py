@@ -454,6 +454,38 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     return out
 
 
+def load_rows_covers(k: torch.Tensor, v: torch.Tensor, k_rows: torch.Tensor, v_rows: torch.Tensor) -> bool:
+    """Whether load_rows takes sources k / v for the cache rows k_rows / v_rows (all [B,T,KH,128]): one dtype and device, 16-byte
+    aligned rows, no shared memory (the source may be a view of a cache), nothing traced."""
+    ts = (k, v, k_rows, v_rows)
+    if not untraced(*ts) or any(t.shape != k_rows.shape or t.dtype != k_rows.dtype or not t.is_cuda or t.device != k_rows.device for t in ts):
+        return False
+    if k_rows.dim() != 4 or k_rows.shape[3] != 128 or k_rows.dtype not in (torch.bfloat16, torch.float16, torch.float32):
+        return False
+    if any(st % (16 // t.element_size()) for t in ts for st in t.stride()[:3]) or any(t.stride(3) != 1 or t.data_ptr() % 16 for t in ts):
+        return False
+    if any(t.is_conj() or t.is_neg() for t in ts):
+        return False
+    dst = {t.untyped_storage().data_ptr() for t in (k_rows, v_rows)}
+    B, T, KH, _ = k_rows.shape
+    distinct = all((KH == 1 or t.stride(2) >= 128) and (T == 1 or t.stride(1) >= 128) and (B == 1 or t.stride(0) >= 128) for t in (k_rows, v_rows))
+    return distinct and k_rows.stride() == v_rows.stride() and k.untyped_storage().data_ptr() not in dst and v.untyped_storage().data_ptr() not in dst
+
+
+def load_rows(k: torch.Tensor, v: torch.Tensor, k_rows: torch.Tensor, v_rows: torch.Tensor, params: Optional[HashParams] = None,
+              codes: Optional[torch.Tensor] = None) -> None:
+    """New keys and values [B,T,KH,128] into the cache rows k_rows / v_rows (views of the caches) and, with `params`, the codes
+    of the keys into codes [B,T,KH,4] (a view of the code cache). See load_rows_covers."""
+    B, T, KH, _ = k_rows.shape
+    _cuda(k, v, k_rows, v_rows)
+    assert params is None or (params.heads == KH and codes.shape == (B, T, KH, 4) and codes.dtype == torch.uint32)
+    kl, vl, cl = _kv_layout(k), _kv_layout(v), _kv_layout(k_rows)
+    check(lib.sl_load_rows(k.data_ptr(), C.byref(kl), v.data_ptr(), C.byref(vl), _dt(k), B, T, KH, k_rows.data_ptr(), v_rows.data_ptr(),
+                           C.byref(cl), params.ref() if params is not None else None, _ptr(codes),
+                           0 if codes is None else _rows_view(codes, 4), _stream()))
+    _count()
+
+
 # ----------------------------------------------------------------------------- attention
 def sparse_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, idx: torch.Tensor,
                        cnt: torch.Tensor, layout: int = GQA_BLOCKED, out: Optional[torch.Tensor] = None,

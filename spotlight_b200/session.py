@@ -90,8 +90,14 @@ class DecodeSession:
         """Copy post-RoPE keys / values [B,T,KH,128] into the caches at [start, start+T) and build
         their codes with the layer's key hash."""
         T = k.shape[1]
-        self.k_cache[layer][:, start:start + T] = k
-        self.v_cache[layer][:, start:start + T] = v
+        k_rows, v_rows = self.k_cache[layer][:, start:start + T], self.v_cache[layer][:, start:start + T]
+        if ops.load_rows_covers(k, v, k_rows, v_rows):
+            ops.load_rows(k, v, k_rows, v_rows, self.hash_k[layer] if codes else None,
+                          self.codes[layer][:, start:start + T] if codes else None)
+            return
+        # host tensors, other dtypes, broadcast or overlapping sources: torch's copy
+        k_rows[:] = k
+        v_rows[:] = v
         if codes:
             ops.hash_encode(self.k_cache[layer][:, start:start + T], self.hash_k[layer],
                             out=self.codes[layer][:, start:start + T])

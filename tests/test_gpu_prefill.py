@@ -77,3 +77,93 @@ def test_the_hook_keeps_the_general_path_for_what_autograd_sees():
         assert not ops.prefill_covers(q, k, v, kc, vc)
     two = kv.expand(2, -1, -1, -1, -1)               # batch rows that share memory
     assert not ops.prefill_covers(q.expand(2, -1, -1, -1), k.expand(2, -1, -1, -1), v.expand(2, -1, -1, -1), two[:, :, :, 0], two[:, :, :, 1])
+
+
+def _hash(kind, heads, gen, dtype=torch.bfloat16):
+    from spotlight_b200 import ops
+    dims, residue = {"linear": ((128, 128), False), "mlp256": ((128, 256, 128), False), "mlp128": ((128, 128, 128), False),
+                     "mlp128_residual": ((128, 128, 128), True)}[kind]
+    ws = [(torch.randn((heads, i, o), generator=gen, device="cuda") * 0.5 / i ** 0.5).to(dtype) for i, o in zip(dims[:-1], dims[1:])]
+    bs = [None if kind == "linear" else (0.1 * torch.randn((heads, o), generator=gen, device="cuda")).to(dtype) for o in dims[1:]]
+    return ops.HashParams(ws, bs, residue)
+
+
+# tile edges (127 .. 129 rows), one tile in flight only, more tiles than CTAs, several batch rows, both cache layouts,
+# a transposed source; kernel 0: by size (the copy kernel below the line), 2: the tensor-core kernel whatever the size
+@pytest.mark.parametrize("kernel", [0, 2])
+@pytest.mark.parametrize("kind", ["linear", "mlp256", "mlp128", "mlp128_residual"])
+@pytest.mark.parametrize("B,T,start,KH,fused", [(1, 127, 0, 8, True), (2, 129, 5, 4, False), (3, 128, 1, 2, True), (1, 5001, 77, 8, True),
+                                                (2, 64, 0, 40, True)])
+def test_load_rows_moves_rows_and_builds_the_codes_of_hash_encode(B, T, start, KH, fused, kind, kernel):
+    from spotlight_b200 import _lib, ops
+    gen = torch.Generator(device="cuda").manual_seed(B * T + KH)
+    kc, vc = _caches(B, start + T + 9, KH, fused, gen)
+    codes = torch.zeros((B, start + T + 9, KH, 4), dtype=torch.int32, device="cuda").view(torch.uint32)
+    k = torch.randn((B, KH, T, 128), generator=gen, device="cuda").bfloat16().transpose(1, 2)       # head-major source
+    v = torch.randn((B, T, KH, 128), generator=gen, device="cuda").bfloat16()
+    h = _hash(kind, KH, gen)
+    k0, v0 = kc.clone(), vc.clone()
+    k0[:, start:start + T], v0[:, start:start + T] = k, v
+    rows = slice(start, start + T)
+    assert ops.load_rows_covers(k, v, kc[:, rows], vc[:, rows])
+    ops.configure(_lib.SL_OPT_HASH_KERNEL, kernel)
+    try:
+        ops.load_rows(k, v, kc[:, rows], vc[:, rows], h, codes[:, rows])
+        want = ops.hash_encode(k0[:, rows], h)
+    finally:
+        ops.configure(_lib.SL_OPT_HASH_KERNEL, 0)
+    torch.cuda.synchronize()
+    assert torch.equal(kc, k0) and torch.equal(vc, v0)
+    got = codes.view(torch.int32)
+    assert torch.equal(got[:, rows], want.view(torch.int32))
+    assert int(got[:, :start].abs().max() if start else 0) == 0 and int(got[:, start + T:].abs().max()) == 0
+    ops.check_status(torch.device("cuda", 0))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_load_rows_other_types(dtype):
+    from spotlight_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    k, v = (torch.randn((2, 131, 3, 128), generator=gen, device="cuda").to(dtype) for _ in range(2))
+    kv = torch.zeros((2, 140, 3, 2, 128), dtype=dtype, device="cuda")
+    codes = torch.zeros((2, 140, 3, 4), dtype=torch.int32, device="cuda").view(torch.uint32)
+    h = _hash("mlp128", 3, gen, dtype)
+    ops.load_rows(k, v, kv[:, 2:133, :, 0], kv[:, 2:133, :, 1], h, codes[:, 2:133])
+    assert torch.equal(kv[:, 2:133, :, 0], k) and torch.equal(kv[:, 2:133, :, 1], v) and int((kv[:, 133:] != 0).sum()) == 0
+    assert torch.equal(codes[:, 2:133].view(torch.int32), ops.hash_encode(k, h).view(torch.int32))
+
+
+def test_load_context_keeps_torchs_copy_for_the_rest():
+    from spotlight_b200.session import DecodeSession, SessionConfig
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    h = [_hash("linear", 2, gen)]
+    s = DecodeSession(SessionConfig(1, 2, 2, 1, 64), h, h)
+    k, v = (torch.randn((1, 20, 2, 128), generator=gen, device="cuda") for _ in range(2))
+    s.load_context(0, k.cpu(), v, 3)                                             # a host tensor, and fp32 into a bf16 cache
+    assert torch.equal(s.k_cache[0][:, 3:23], k.bfloat16()) and torch.equal(s.v_cache[0][:, 3:23], v.bfloat16())
+    s.load_context(0, s.k_cache[0][:, 3:13], s.v_cache[0][:, 3:13], 30)          # a view of the cache itself
+    assert torch.equal(s.k_cache[0][:, 30:40], k.bfloat16()[:, :10]) and torch.equal(s.codes[0][:, 30:40].view(torch.int32), s.codes[0][:, 3:13].view(torch.int32))
+    s.load_context(0, k[:, :1, :1].bfloat16(), v[:, :1].bfloat16(), 50)          # one head for both
+    assert torch.equal(s.k_cache[0][:, 50, 1], s.k_cache[0][:, 50, 0])
+
+
+def test_the_hash_kernels_silu_is_the_accurate_formula_for_every_bf16():
+    """Every finite bf16 through the tcgen05 kernel's activation: with an identity first layer, hidden value j of a row is
+    silu(x_j); +-identity in the second layer and torch's value (fp32 x / (1 + exp(-x)), rounded once) taken off as the bias
+    leave a sign bit exactly where the hidden value is larger (smaller) than that."""
+    from spotlight_b200 import _lib, ops
+    bits = torch.arange(65536, dtype=torch.int32)
+    x = bits.to(torch.int16).view(torch.bfloat16).view(512, 128).cuda()
+    x = torch.where(torch.isfinite(x), x, torch.zeros_like(x))
+    ref = torch.nn.functional.silu(x)
+    rows = x[None, None].expand(1, 64, -1, -1).contiguous()
+    eye = torch.eye(128, device="cuda").bfloat16().expand(512, 128, 128)
+    ops.configure(_lib.SL_OPT_HASH_KERNEL, 2)
+    try:
+        for sign in (1, -1):
+            codes = ops.hash_encode(rows, ops.HashParams([eye, sign * eye], [None, -sign * ref]))
+            assert int(codes.view(torch.int32).ne(0).sum()) == 0, f"sign {sign}"
+        codes = ops.hash_encode(rows, ops.HashParams([eye, eye], [None, -ref + 2.0 ** -120]))        # the test does see a difference
+        assert int(codes.view(torch.int32).ne(0).sum()) > 0
+    finally:
+        ops.configure(_lib.SL_OPT_HASH_KERNEL, 0)
