@@ -290,6 +290,10 @@ int sl_sparse_attn_decode_ex(const void* d_q, const void* d_k, const void* d_v, 
                              const int32_t* d_idx, int idx_capacity, const int32_t* d_cnt, int B, int KH, int QH,
                              int gqa_layout, void* d_out, float* d_lse, void* d_workspace, size_t workspace_bytes,
                              void* stream);
+/* The same over EVERY key 0 .. n-1, without a list (layers that attend to all keys). */
+int sl_dense_attn_decode(const void* d_q, const void* d_k, const void* d_v, int dtype, const sl_kv_layout* kv, int n, int B,
+                         int KH, int QH, int gqa_layout, void* d_out, float* d_lse, void* d_workspace,
+                         size_t workspace_bytes, void* stream);
 
 /* sl_sparse_attn_decode for callers that may not allocate device memory where they run attention
  * (an engine whose memory pool took all of HBM at start-up; a decode loop in which cudaMalloc and
@@ -457,6 +461,10 @@ typedef struct {
     void* d_lru_workspace; size_t lru_workspace_bytes;
 } sl_decode_step_args;
 int sl_decode_step(const sl_decode_step_args* args, int64_t pos, void* stream);
+/* The same for tables that keep a clock of their own: lru_steps [layers] (host memory) are the clocks, each advanced by one as
+ * its layer is launched; d_lru_status [layers] (host array of device words) takes the tables' status instead of d_status.
+ * Either may be NULL (the position is the clock; d_status). */
+int sl_decode_step_lru(const sl_decode_step_args* args, int64_t pos, int32_t* lru_steps, int32_t* const* d_lru_status, void* stream);
 
 /* sl_decode_step with the position in DEVICE memory, so that ONE captured sequence of launches (a CUDA
  * graph) serves every token of a decode loop: the token sits at *d_pos, the context is *d_pos + 1 keys,

@@ -95,6 +95,7 @@ SIGNATURES = {
     "sl_sparse_attn_workspace_bytes": (_Z, [_I, _I, _I]),
     "sl_sparse_attn_decode": (_I, [_P, _P, _P, _I, _L, _P, _I, _P, _I, _I, _I, _I, _P, _P, _P, _Z, _P]),
     "sl_sparse_attn_decode_ex": (_I, [_P, _P, _P, _I, _KV, _P, _I, _P, _I, _I, _I, _I, _P, _P, _P, _Z, _P]),
+    "sl_dense_attn_decode": (_I, [_P, _P, _P, _I, _KV, _I, _I, _I, _I, _I, _P, _P, _P, _Z, _P]),
     "sl_sparse_attn_decode_fill": (_I, [_P, _P, _P, _I, _KV, _P, _I, _P, _I, _I, _I, _I, _P, _P, _P, _Z, C.POINTER(AttnFill), _P]),
     "sl_lru_probe": (_I, [_P, _I, _P, _I, _I, _I, _P, _P, _KV, _I, _P, _L, _P, _P, _I, _P, _P, _P, _P, _Z, _P]),
     "sl_lru_evict": (_I, [_P, _I, _P, _I, _I, _P, _P, _KV, _I, _P, _P, _KV, _I, _P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _Z, _P]),
@@ -106,6 +107,7 @@ SIGNATURES = {
     "sl_lru_update_ex": (_I, [_P, _I, _P, _I, _I, _P, _P, _KV, _I, _P, _P, _KV, _I, _P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _Z, _P]),
     "sl_gather_rows": (_I, [_P, _L, _I, _P, _I, _I, _I, _I, _P, _P]),
     "sl_decode_step": (_I, [C.POINTER(DecodeStepArgs), _L, _P]),
+    "sl_decode_step_lru": (_I, [C.POINTER(DecodeStepArgs), _L, C.POINTER(_I), _PP, _P]),
     "sl_decode_step_dev": (_I, [C.POINTER(DecodeStepArgs), C.POINTER(DecodeDev), _P]),
     "sl_scan_topk_sharded_slot_bytes": (_Z, [_I, _I, _I]),
     "sl_scan_topk_sharded": (_I, [_P, _P, _L, _I, _L, _L, _L, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P, _Z, C.POINTER(_P),

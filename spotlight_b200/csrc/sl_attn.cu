@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(AT, (G * (16 / sizeof(T)) > 32) ? 1 : 2) spars
     const int sp = blockIdx.x, h = blockIdx.y, b = blockIdx.z, KH = a.KH;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int sub = lane % LPR, rs = lane / LPR;
-    const int n = a.cnt[b * KH + h];
+    const int n = a.idx ? a.cnt[b * KH + h] : a.cap;
     const int per = (n + a.splits - 1) / a.splits;
     const int lo = min(n, sp * per), hi = min(n, lo + per);
     const int* list = a.idx + ((long long)b * KH + h) * a.cap;
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(AT, (G * (16 / sizeof(T)) > 32) ? 1 : 2) spars
         const bool ok = it < nit && j < hi;
         okb[slot] = ok;
         if (ok) {
-            const long long tok = list[j];
+            const long long tok = a.idx ? list[j] : j;
             kbuf[slot] = sl::ld_gather_v4(kb + tok * row_stride);
             vbuf[slot] = sl::ld_gather_v4(vb + tok * row_stride);
         }
@@ -305,8 +305,8 @@ extern "C" size_t sl_sparse_attn_workspace_bytes(int B, int KH, int QH) {
 static int attn_decode(const void* d_q, const void* d_k, const void* d_v, int dtype, const sl_kv_layout* kv,
                        const int32_t* d_idx, int idx_capacity, const int32_t* d_cnt, int B, int KH, int QH,
                        int gqa_layout, void* d_out, float* d_lse, void* d_workspace, size_t workspace_bytes,
-                       const sl_attn_fill* fill, void* stream) {
-    SL_REQUIRE(d_q && d_k && d_v && kv && d_idx && d_cnt && d_out && d_workspace, SL_EINVAL, "sl_sparse_attn_decode: null pointer");
+                       const sl_attn_fill* fill, void* stream, bool dense = false) {
+    SL_REQUIRE(d_q && d_k && d_v && kv && (dense || (d_idx && d_cnt)) && d_out && d_workspace, SL_EINVAL, "sl_sparse_attn_decode: null pointer");
     SL_REQUIRE(B > 0 && KH > 0 && QH > 0 && QH % KH == 0 && idx_capacity > 0, SL_ESHAPE, "sl_sparse_attn_decode: bad shape");
     SL_REQUIRE(B <= 65535 && KH <= 65535, SL_ESHAPE, "sl_sparse_attn_decode: B or KH > 65535");
     SL_REQUIRE(gqa_layout == SL_GQA_INTERLEAVED || gqa_layout == SL_GQA_BLOCKED, SL_EINVAL,
@@ -365,6 +365,13 @@ extern "C" int sl_sparse_attn_decode_ex(const void* d_q, const void* d_k, const 
                                         void* stream) {
     return attn_decode(d_q, d_k, d_v, dtype, kv, d_idx, idx_capacity, d_cnt, B, KH, QH, gqa_layout, d_out, d_lse, d_workspace,
                        workspace_bytes, nullptr, stream);
+}
+
+extern "C" int sl_dense_attn_decode(const void* d_q, const void* d_k, const void* d_v, int dtype, const sl_kv_layout* kv, int n, int B,
+                                    int KH, int QH, int gqa_layout, void* d_out, float* d_lse, void* d_workspace,
+                                    size_t workspace_bytes, void* stream) {
+    return attn_decode(d_q, d_k, d_v, dtype, kv, nullptr, n, nullptr, B, KH, QH, gqa_layout, d_out, d_lse, d_workspace, workspace_bytes,
+                       nullptr, stream, true);
 }
 
 extern "C" int sl_sparse_attn_decode_fill(const void* d_q, void* d_k_resident, void* d_v_resident, int dtype,

@@ -12,7 +12,7 @@ struct AttnArgs {
     long long tok_stride;          // elements between the rows of consecutive keys (KH * 128 for [B,N,KH,128])
     long long head_stride;         // elements between the rows of consecutive kv heads of one key (128)
     int kv_div;                    // list heads (entries of idx/cnt per batch row) per kv head of the caches (1)
-    const int* idx; int cap; const int* cnt;
+    const int* idx; int cap; const int* cnt;      // idx null: no list, every key 0 .. cap - 1
     int B, KH, layout, splits;
     void* out; float* lse;
     float* part;                   // [B*KH][splits][G][130]: o[128], m, l

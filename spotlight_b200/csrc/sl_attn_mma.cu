@@ -49,7 +49,9 @@ __device__ __forceinline__ unsigned swz(int r, int c) { return (unsigned)(r * 25
 // distributed shared memory (no partials in global memory, no merge kernel).
 // FILL: the caches are the resident buffers of an LRU table and the list holds slots; rows of entries -(slot + 1) come
 // from the backing store and are written into their slot from shared memory once they have landed.
-template <bool HI, int MW, bool CL, bool FILL>
+// DENSE: no list, the entries are the keys 0 .. cap - 1 themselves (layers that attend to every key: 32 000 keys of 8 heads cost
+// two launches and 2 MB of indices per layer before).
+template <bool HI, int MW, bool CL, bool FILL, bool DENSE>
 __global__ void __launch_bounds__(MW * 32, 8 / MW) sparse_attn_mma_kernel(const AttnArgs a, const int G) {
     constexpr int MT = MW * 32;
     extern __shared__ __align__(128) unsigned char ring[];          // [MW][ST][K 4 KB | V 4 KB]; reused by the epilogue
@@ -60,7 +62,7 @@ __global__ void __launch_bounds__(MW * 32, 8 / MW) sparse_attn_mma_kernel(const 
     const int sp = blockIdx.x, h = blockIdx.y, b = blockIdx.z, KH = a.KH;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int grp = lane >> 2, tig = lane & 3;
-    const int* list = a.idx + ((long long)b * KH + h) * a.cap;
+    const int* list = DENSE ? nullptr : a.idx + ((long long)b * KH + h) * a.cap;
     // The list length decides which tiles are this CTA's, and the list entries decide which rows to fetch: two dependent
     // trips to memory before the first gather. The lists of a decode step are (nearly) as long as their capacity, so the
     // first ST-1 tiles are read as if the length were the capacity, together with the length; they are used when the
@@ -71,13 +73,13 @@ __global__ void __launch_bounds__(MW * 32, 8 / MW) sparse_attn_mma_kernel(const 
     {
         const int t_spec = min(cap_tiles, sp * per_spec) + warp;
 #pragma unroll
-        for (int s = 0; s < ST - 1; ++s) spec[s] = __ldg(list + min((t_spec + s * MW) * 16 + (lane & 15), a.cap - 1));
+        for (int s = 0; s < ST - 1; ++s) spec[s] = DENSE ? 0 : __ldg(list + min((t_spec + s * MW) * 16 + (lane & 15), a.cap - 1));
     }
-    const int n = a.cnt[b * KH + h];
+    const int n = DENSE ? a.cap : a.cnt[b * KH + h];
     const int ntiles = (n + 15) >> 4;
     const int per = (ntiles + a.splits - 1) / a.splits;
     const int tile_lo = min(ntiles, sp * per), tile_hi = min(ntiles, tile_lo + per);
-    const bool spec_ok = per == per_spec;               // then tile_lo is the speculated one as well
+    const bool spec_ok = !DENSE && per == per_spec;               // then tile_lo is the speculated one as well
     const long long row_stride = a.tok_stride;
     const long long hoff = (long long)b * a.kv_b + (long long)(h / a.kv_div) * a.head_stride;
     const __nv_bfloat16* kb = reinterpret_cast<const __nv_bfloat16*>(a.k) + hoff + (lane & 15) * 8;
@@ -89,7 +91,7 @@ __global__ void __launch_bounds__(MW * 32, 8 / MW) sparse_attn_mma_kernel(const 
     const __nv_bfloat16* vbb = FILL ? reinterpret_cast<const __nv_bfloat16*>(a.v_back) + bhoff + (lane & 15) * 8 : nullptr;
 
     // one tile = list entries [16 t, 16 t + 16); lane l < 16 fetches entry l (clamped to the last one)
-    auto entry = [&](int t) -> int { return list[min(t * 16 + (lane & 15), n - 1)]; };
+    auto entry = [&](int t) -> int { const int j = min(t * 16 + (lane & 15), n - 1); return DENSE ? j : list[j]; };
     // a half-warp copies one 256-byte row per step: 8 steps for K, 8 for V
     // fill mode: the key of list entry 16 t + lane (read a tile ahead, like the entry itself)
     auto key_of = [&](int t) -> int { return FILL ? toks[min(t * 16 + (lane & 15), n - 1)] : 0; };
@@ -374,10 +376,10 @@ void set_attn_warps(int v) { g_attn_warps = v; }
 void set_attn_cluster(int v) { g_attn_cluster = v; }
 static bool fat_ctas(int B, int KH) { return g_attn_warps ? g_attn_warps == 8 : B * KH <= sm_count(); }
 
-template <bool HI, int MW, bool FILL>
+template <bool HI, int MW, bool FILL, bool DENSE>
 static cudaError_t cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attrs, int cs, int KH, int B, cudaStream_t s) {
     const size_t ring_bytes = (size_t)MW * ST * STAGE_BYTES;
-    const void* fn = reinterpret_cast<const void*>(sparse_attn_mma_kernel<HI, MW, true, FILL>);
+    const void* fn = reinterpret_cast<const void*>(sparse_attn_mma_kernel<HI, MW, true, FILL, DENSE>);
     cudaError_t e = ensure_dyn_smem(fn, ring_bytes);
     if (e != cudaSuccess) return e;
     static bool allowed = false;                       // per instantiation: clusters of more than 8 CTAs are an opt-in
@@ -410,8 +412,8 @@ static int max_clusters(int cs) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attrs[2];
         int n = 0;
-        if (cluster_config<false, MW, false>(cfg, attrs, cs, 1, 1, nullptr) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(sparse_attn_mma_kernel<false, MW, true, false>), &cfg) != cudaSuccess) {
+        if (cluster_config<false, MW, false, false>(cfg, attrs, cs, 1, 1, nullptr) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(sparse_attn_mma_kernel<false, MW, true, false, false>), &cfg) != cudaSuccess) {
             cudaGetLastError();
             n = 0;
         }
@@ -448,33 +450,34 @@ int attn_mma_splits(int B, int KH, int cap, int reserve_sms) {
     return s;
 }
 
-template <bool HI, int MW, bool FILL>
+template <bool HI, int MW, bool FILL, bool DENSE>
 static int launch_one(const AttnArgs& a, int G, cudaStream_t s) {
     const size_t ring_bytes = (size_t)MW * ST * STAGE_BYTES;
     if (use_cluster(a.B, a.KH, a.splits)) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attrs[2];
-        SL_CUDA_OK((cluster_config<HI, MW, FILL>(cfg, attrs, a.splits, a.KH, a.B, s)));
-        SL_CUDA_OK(cudaLaunchKernelEx(&cfg, sparse_attn_mma_kernel<HI, MW, true, FILL>, a, G));
+        SL_CUDA_OK((cluster_config<HI, MW, FILL, DENSE>(cfg, attrs, a.splits, a.KH, a.B, s)));
+        SL_CUDA_OK(cudaLaunchKernelEx(&cfg, sparse_attn_mma_kernel<HI, MW, true, FILL, DENSE>, a, G));
         return SL_OK;
     }
     dim3 grid((unsigned)a.splits, (unsigned)a.KH, (unsigned)a.B);
-    SL_CUDA_OK(ensure_dyn_smem(reinterpret_cast<const void*>(sparse_attn_mma_kernel<HI, MW, false, FILL>), ring_bytes));
-    SL_CUDA_OK(launch_kernel(sparse_attn_mma_kernel<HI, MW, false, FILL>, grid, dim3(MW * 32), ring_bytes, s, false, a, G));
+    SL_CUDA_OK(ensure_dyn_smem(reinterpret_cast<const void*>(sparse_attn_mma_kernel<HI, MW, false, FILL, DENSE>), ring_bytes));
+    SL_CUDA_OK(launch_kernel(sparse_attn_mma_kernel<HI, MW, false, FILL, DENSE>, grid, dim3(MW * 32), ring_bytes, s, false, a, G));
     if (a.splits > 1) return launch_attn_merge(a, G, SL_BF16, s);
     return SL_OK;
 }
 
-template <bool FILL>
+template <bool FILL, bool DENSE>
 static int launch_by_shape(const AttnArgs& a, int G, cudaStream_t s) {
-    if (fat_ctas(a.B, a.KH)) return G > 8 ? launch_one<true, 8, FILL>(a, G, s) : launch_one<false, 8, FILL>(a, G, s);
-    return G > 8 ? launch_one<true, 4, FILL>(a, G, s) : launch_one<false, 4, FILL>(a, G, s);
+    if (fat_ctas(a.B, a.KH)) return G > 8 ? launch_one<true, 8, FILL, DENSE>(a, G, s) : launch_one<false, 8, FILL, DENSE>(a, G, s);
+    return G > 8 ? launch_one<true, 4, FILL, DENSE>(a, G, s) : launch_one<false, 4, FILL, DENSE>(a, G, s);
 }
 
 int attn_cluster_capacity(int warps, int cs) { return warps == 8 ? max_clusters<8>(cs) : max_clusters<4>(cs); }
 
 int launch_attn_mma(const AttnArgs& a, int G, cudaStream_t s) {
-    return a.tok ? launch_by_shape<true>(a, G, s) : launch_by_shape<false>(a, G, s);
+    if (!a.idx) return launch_by_shape<false, true>(a, G, s);
+    return a.tok ? launch_by_shape<true, false>(a, G, s) : launch_by_shape<false, false>(a, G, s);
 }
 
 }  // namespace sl

@@ -12,7 +12,9 @@ __global__ void advance_pos_kernel(long long* pos) {
     *pos += 1;
 }
 
-int run_layers(const sl_decode_step_args* a, int64_t pos, const sl_decode_dev* dev, void* stream) {
+// lru_steps / lru_status: per layer, the clock of its LRU table (advanced as the layer is launched; null: the position is
+// the clock) and its own status word (null: a->d_status)
+int run_layers(const sl_decode_step_args* a, int64_t pos, const sl_decode_dev* dev, int32_t* lru_steps, int32_t* const* lru_status, void* stream) {
     SL_REQUIRE(a != nullptr, SL_EINVAL, "sl_decode_step: null argument block");
     SL_REQUIRE(a->layers > 0 && a->d_q && a->d_out && a->hash_q && a->d_code_cache && a->d_k_cache && a->d_v_cache,
                SL_EINVAL, "sl_decode_step: null pointer table");
@@ -55,14 +57,17 @@ int run_layers(const sl_decode_step_args* a, int64_t pos, const sl_decode_dev* d
         if (a->lru) {
             const sl_lru_layer& t = a->lru[l];
             const sl_kv_layout res = {a->lru_batch_stride, a->lru_token_stride, a->lru_head_stride, 1};
+            const int step = lru_steps ? lru_steps[l] : (int)pos;
+            int32_t* status = lru_status ? lru_status[l] : a->d_status;
             const int64_t* d_step = dev ? reinterpret_cast<const int64_t*>(dp.d_pos) : nullptr;
             if (sl::lru_fused_fill() && a->dtype == SL_BF16 && a->QH / a->KH <= 16) {
                 // the attention launch fetches the rows of the misses itself and fills their slots on the way
                 rc = sl_lru_update_deferred(a->d_idx, a->idx_capacity, a->d_cnt, a->B, a->KH, 2, t.d_k_resident, t.d_v_resident,
-                                            &res, a->lru_slots, t.d_tok2slot, a->lru_n_max, t.d_slot2tok, t.d_last_used, (int)pos,
-                                            d_step, a->d_slots, t.d_stats, a->d_status, a->d_lru_workspace,
+                                            &res, a->lru_slots, t.d_tok2slot, a->lru_n_max, t.d_slot2tok, t.d_last_used, step,
+                                            d_step, a->d_slots, t.d_stats, status, a->d_lru_workspace,
                                             a->lru_workspace_bytes, stream);
                 if (rc) return rc;
+                if (lru_steps) ++lru_steps[l];
                 const sl_attn_fill fill = {a->d_idx, a->d_k_cache[l], a->d_v_cache[l], kv};
                 rc = sl_sparse_attn_decode_fill(a->d_q_rot, t.d_k_resident, t.d_v_resident, a->dtype, &res, a->d_slots,
                                                 a->idx_capacity, a->d_cnt, a->B, a->KH, a->QH, a->gqa_layout, a->d_out[l], nullptr,
@@ -70,9 +75,10 @@ int run_layers(const sl_decode_step_args* a, int64_t pos, const sl_decode_dev* d
             } else {
                 rc = sl_lru_update_ex(a->d_idx, a->idx_capacity, a->d_cnt, a->B, a->KH, a->d_k_cache[l], a->d_v_cache[l], &kv,
                                       a->dtype == SL_F32 ? 4 : 2, t.d_k_resident, t.d_v_resident, &res, a->lru_slots, t.d_tok2slot,
-                                      a->lru_n_max, t.d_slot2tok, t.d_last_used, (int)pos, d_step, a->d_slots, t.d_stats,
-                                      a->d_status, a->d_lru_workspace, a->lru_workspace_bytes, stream);
+                                      a->lru_n_max, t.d_slot2tok, t.d_last_used, step, d_step, a->d_slots, t.d_stats,
+                                      status, a->d_lru_workspace, a->lru_workspace_bytes, stream);
                 if (rc) return rc;
+                if (lru_steps) ++lru_steps[l];
                 rc = sl_sparse_attn_decode_ex(a->d_q_rot, t.d_k_resident, t.d_v_resident, a->dtype, &res, a->d_slots,
                                               a->idx_capacity, a->d_cnt, a->B, a->KH, a->QH, a->gqa_layout, a->d_out[l], nullptr,
                                               a->d_attn_workspace, a->attn_workspace_bytes, stream);
@@ -93,10 +99,14 @@ int run_layers(const sl_decode_step_args* a, int64_t pos, const sl_decode_dev* d
 }  // namespace
 
 extern "C" int sl_decode_step(const sl_decode_step_args* a, int64_t pos, void* stream) {
-    return run_layers(a, pos, nullptr, stream);
+    return run_layers(a, pos, nullptr, nullptr, nullptr, stream);
+}
+
+extern "C" int sl_decode_step_lru(const sl_decode_step_args* a, int64_t pos, int32_t* lru_steps, int32_t* const* d_lru_status, void* stream) {
+    return run_layers(a, pos, nullptr, lru_steps, d_lru_status, stream);
 }
 
 extern "C" int sl_decode_step_dev(const sl_decode_step_args* a, const sl_decode_dev* dev, void* stream) {
     SL_REQUIRE(dev != nullptr, SL_EINVAL, "sl_decode_step_dev: null device-position block");
-    return run_layers(a, dev->max_context - 1, dev, stream);
+    return run_layers(a, dev->max_context - 1, dev, nullptr, nullptr, stream);
 }

@@ -103,8 +103,33 @@ class LayerState:
         self.kv = torch.empty((batch, capacity, kv_heads, 2, 128), dtype=dtype, device=device)
         self.codes = torch.empty((batch, capacity, list_heads or kv_heads, 4), dtype=torch.uint32, device=device)
         self.length = 0
-        self.last_idx = None
-        self.last_cnt = None
+        self._last = (None, None)
+
+    # the keys the last decode step attended to: idx int32 [B,LH,cap] ascending, cnt int32 [B,LH]; after a dense layer
+    # (which needs no list) made when they are asked for
+    def _attended(self):
+        if isinstance(self._last, int):
+            n, dev = self._last, self.kv.device
+            heads = (self.kv.shape[0], self.kv.shape[2])
+            self._last = (torch.arange(n, dtype=torch.int32, device=dev).expand(*heads, n).contiguous(),
+                          torch.full(heads, n, dtype=torch.int32, device=dev))
+        return self._last
+
+    @property
+    def last_idx(self):
+        return self._attended()[0]
+
+    @last_idx.setter
+    def last_idx(self, idx):
+        self._last = (idx, self._attended()[1])
+
+    @property
+    def last_cnt(self):
+        return self._attended()[1]
+
+    @last_cnt.setter
+    def last_cnt(self, cnt):
+        self._last = (self._attended()[0], cnt)
 
     @property
     def k(self):
@@ -233,27 +258,38 @@ def self_attn_forward(self, hidden_states: torch.Tensor, kv_cache: Optional[Laye
     pos = st.length
     cos, sin = _rope_table(pos + 1, theta, q.dtype, q.device)
     cos, sin = cos[pos], sin[pos]
+    k_cache, v_cache = st.k, st.v
+    if hashed and not per_q and type(kw["mask_out"]) in (int, float) and type(kw.get("min_remain", 20)) is int:
+        n = pos + 1
+        keep = budget(n, kw["mask_out"], kw.get("min_remain", 20))
+        o, idx, cnt = ops.decode_layer(q[:, 0], k[:, 0], v[:, 0], self._hash_q_params(), self._hash_k_params(), pos, st.codes, k_cache, v_cache,
+                                       cos, sin, keep, kw["mask_out"], kw.get("min_remain", 20), int(kw.get("sink", 4)),
+                                       int(kw.get("recent", 64)), GQA_BLOCKED)
+        st.length = n
+        st._last = (idx, cnt)
+        return self.o_proj(o.view(B, 1, num_heads * head_dim)), st
     if hashed and per_q:
         # codes of the new key under every query head's parameters; its K/V rows are appended per KV head
         q_rot, q_codes = ops.decode_prepare(q[:, 0], k[:, 0].repeat_interleave(G, dim=1), None, self._hash_q_params(),
                                             self._hash_q_params(), pos, code_cache=st.codes, cos=cos, sin=sin)
-        st.k[:, pos] = _rotate(k[:, 0], cos, sin)
-        st.v[:, pos] = v[:, 0]
+        k_cache[:, pos] = _rotate(k[:, 0], cos, sin)
+        v_cache[:, pos] = v[:, 0]
     else:
         q_rot, q_codes = ops.decode_prepare(
             q[:, 0], k[:, 0], v[:, 0], self._hash_q_params() if hashed else _IDENTITY_HASH.get(num_heads, q),
             self._hash_k_params() if hashed else _IDENTITY_HASH.get(num_kv_heads, q), pos,
-            code_cache=st.codes, k_cache=st.k, v_cache=st.v, cos=cos, sin=sin)
+            code_cache=st.codes, k_cache=k_cache, v_cache=v_cache, cos=cos, sin=sin)
     st.length = n = pos + 1
+    if not pruned:
+        o = ops.dense_attn_decode(q_rot, k_cache, v_cache, n, GQA_BLOCKED)
+        st._last = n
+        return self.o_proj(o.view(B, 1, num_heads * head_dim)), st
     if hashed:
         idx, cnt = _select(self, q_rot, q_codes, st, n, lh)
-    elif pruned:
-        idx, cnt = self.select_indices(q_rot, st, n)          # another index source (e.g. the exact top-k)
     else:
-        idx = torch.arange(n, dtype=torch.int32, device=q.device).expand(B, num_kv_heads, n).contiguous()
-        cnt = torch.full((B, num_kv_heads), n, dtype=torch.int32, device=q.device)
-    st.last_idx, st.last_cnt = idx, cnt
-    o = ops.sparse_attn_decode(q_rot, st.k[:, :n], st.v[:, :n], idx, cnt, GQA_BLOCKED)
+        idx, cnt = self.select_indices(q_rot, st, n)          # another index source (e.g. the exact top-k)
+    st._last = (idx, cnt)
+    o = ops.sparse_attn_decode(q_rot, k_cache[:, :n], v_cache[:, :n], idx, cnt, GQA_BLOCKED)
     return self.o_proj(o.view(B, 1, num_heads * head_dim)), st
 
 

@@ -44,7 +44,7 @@ def _cuda(*tensors: torch.Tensor) -> torch.device:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())     # torch.cuda.current_stream() without its Stream object
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -516,6 +516,67 @@ def sparse_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
                                        out.data_ptr(), _ptr(lse), ws.data_ptr(), ws.numel(), _stream()))
     _count()
     return (out, lse) if return_lse else out
+
+
+def dense_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, n: int, layout: int = GQA_BLOCKED) -> torch.Tensor:
+    """sparse_attn_decode over the keys 0 .. n-1 of the caches, without an index list."""
+    B, QH, D = q.shape
+    KH = k_cache.shape[2]
+    assert D == 128 and k_cache.dtype == q.dtype and v_cache.dtype == q.dtype and QH % KH == 0 and n <= k_cache.shape[1]
+    dev = _cuda(q, k_cache, v_cache)
+    q = q.contiguous()
+    kv, kv2 = _kv_layout(k_cache), _kv_layout(v_cache)
+    assert (kv2.batch_stride, kv2.token_stride, kv2.head_stride) == (kv.batch_stride, kv.token_stride, kv.head_stride)
+    out = torch.empty_like(q)
+    ws, _ = workspaces.get("attn", dev, lib.sl_sparse_attn_workspace_bytes(B, KH, QH), (B, KH, QH))
+    check(lib.sl_dense_attn_decode(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), _dt(q), C.byref(kv), n, B, KH, QH, layout,
+                                   out.data_ptr(), None, ws.data_ptr(), ws.numel(), _stream()))
+    _count()
+    return out
+
+
+def decode_layer(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, hash_q: HashParams, hash_k: HashParams, pos: int, code_cache: torch.Tensor,
+                 k_cache: torch.Tensor, v_cache: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, keep: int, mask_out: float,
+                 min_remain: int, sink: int, recent: int, layout: int = GQA_BLOCKED):
+    """decode_prepare, scan_topk and sparse_attn_decode of one layer and token in ONE call into the library: q [B,QH,128], k / v
+    [B,KH,128]; row `pos` of the full caches is written, keys 0 .. pos are scanned. `keep` is budget(pos + 1, mask_out, min_remain),
+    which the library evaluates again by the same rule. Returns (out [B,QH,128], idx, cnt)."""
+    B, QH, D = q.shape
+    KH, n = k.shape[1], pos + 1
+    assert D == 128
+    dev = _cuda(q, code_cache)
+    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+    assert code_cache.shape[0] == B and code_cache.shape[2:] == (KH, 4)
+    assert pos < code_cache.shape[1], "code cache is full"
+    assert pos < k_cache.shape[1], "kv cache is full"
+    assert k_cache.dtype == q.dtype and v_cache.dtype == q.dtype
+    kv, kv2 = _kv_layout(k_cache), _kv_layout(v_cache)
+    assert (kv2.batch_stride, kv2.token_stride, kv2.head_stride) == (kv.batch_stride, kv.token_stride, kv.head_stride)
+    cap = max(1, min(n, keep + sink + recent))
+    idx = torch.empty((B, KH, cap), dtype=torch.int32, device=dev)
+    cnt = torch.empty((B, KH), dtype=torch.int32, device=dev)
+    q_rot, out = torch.empty_like(q), torch.empty_like(q)
+    q_codes = torch.empty((B, QH, 4), dtype=torch.int32, device=dev)
+    shape = (B, KH, QH)
+    sw, status = workspaces.get("scan", dev, lib.sl_scan_topk_workspace_bytes(B, n, KH, QH), shape)
+    aw, _ = workspaces.get("attn", dev, lib.sl_sparse_attn_workspace_bytes(B, KH, QH), shape)
+    P = C.c_void_p * 1
+    a = _lib.DecodeStepArgs()
+    a.B, a.QH, a.KH, a.layers, a.dtype, a.gqa_layout = B, QH, KH, 1, _dt(q), layout
+    a.sink, a.recent, a.min_remain, a.mask_out = sink, recent, min_remain, mask_out
+    a.code_batch_stride = _rows_view(code_cache, 4)
+    a.kv_batch_stride, a.kv_token_stride, a.kv_head_stride = kv.batch_stride, kv.token_stride, kv.head_stride
+    a.d_q, a.d_k, a.d_v, a.d_out = P(q.data_ptr()), P(k.data_ptr()), P(v.data_ptr()), P(out.data_ptr())
+    a.hash_q, a.hash_k = C.pointer(hash_q.struct), C.pointer(hash_k.struct)
+    a.d_code_cache, a.d_k_cache, a.d_v_cache = P(code_cache.data_ptr()), P(k_cache.data_ptr()), P(v_cache.data_ptr())
+    a.d_cos, a.d_sin = cos.data_ptr(), sin.data_ptr()
+    a.d_q_rot, a.d_q_codes = q_rot.data_ptr(), q_codes.data_ptr()
+    a.d_idx, a.idx_capacity, a.d_cnt = idx.data_ptr(), cap, cnt.data_ptr()
+    a.d_scan_workspace, a.scan_workspace_bytes, a.d_status = sw.data_ptr(), sw.numel(), status.data_ptr()
+    a.d_attn_workspace, a.attn_workspace_bytes = aw.data_ptr(), aw.numel()
+    check(lib.sl_decode_step(C.byref(a), pos, _stream()))
+    _count(3)
+    return out, idx, cnt
 
 
 def sparse_attn_decode_fill(q: torch.Tensor, table: "LruTable", slots: torch.Tensor, idx: torch.Tensor, cnt: torch.Tensor,

@@ -152,37 +152,114 @@ class DecodeSession:
                                        self.cnt, c.layout, out=self.out[layer])
 
     def step(self, pos: int, stage: Optional[str] = None):
+        """All layers, in one call into the library where that does what the calls of layer_step would do, one after another."""
+        if stage is None and self._one_call(pos):
+            self._step_in_one_call(pos)
+            return
         for layer in range(self.cfg.layers):
             self.layer_step(layer, pos, stage)
 
-    def _native_args(self):
+    def _one_call(self, pos: int) -> bool:
+        """Whether sl_decode_step_lru serves `step(pos)`: the position is inside the caches, no dense layers, layer_step is this
+        class's, and the buffers (which a caller may have exchanged) still have one geometry for all layers."""
+        c = self.cfg
+        if c.fix_layers or not 0 <= pos < c.capacity or type(self).layer_step is not DecodeSession.layer_step or "layer_step" in self.__dict__:
+            return False
+        L, dt = c.layers, self.q_in.dtype
+        if not (len(self.codes) == len(self.k_cache) == len(self.v_cache) == len(self.hash_q) == len(self.hash_k) == L):
+            return False
+        ks, cs, kn, cn = self.k_cache[0].stride(), self.codes[0].stride(), self.k_cache[0].shape, self.codes[0].shape
+        if kn[1] <= pos or cn[1] <= pos or cn[2:] != (c.kv_heads, 4) or cs[1:] != (c.kv_heads * 4, 4, 1) or ks[3] != 1:
+            return False
+        for k, v, codes in zip(self.k_cache, self.v_cache, self.codes):
+            if k.stride() != ks or v.stride() != ks or codes.stride() != cs or k.shape != kn or v.shape != kn or codes.shape != cn \
+                    or k.dtype != dt or v.dtype != dt or not k.is_cuda:
+                return False
+        for t, h in ((self.q_in, c.q_heads), (self.k_in, c.kv_heads), (self.v_in, c.kv_heads), (self.out, c.q_heads)):
+            if t.shape != (L, c.batch, h, 128) or t.dtype != dt or not t.is_contiguous() or not t.is_cuda:
+                return False
+        if self.lru is not None and self.use_lru:
+            rs = self.lru[0].k.stride()
+            if len(self.lru) != L or any((t.C, t.n_max, t.k.stride(), t.v.stride()) != (c.lru_slots, c.capacity, rs, rs) for t in self.lru):
+                return False
+        return self.idx.is_contiguous() and self.idx.shape[:2] == (c.batch, c.kv_heads)
+
+    def _step_in_one_call(self, pos: int):
         import ctypes as C
+        from . import _lib
+        c, L, n = self.cfg, self.cfg.layers, pos + 1
+        ops._cuda(self.q_in)
+        a, keep = self._step_args()                  # from the buffers as they are now
+        shape = (c.batch, c.kv_heads, c.q_heads)
+        sw, status = ops.workspaces.get("scan", self.device, _lib.lib.sl_scan_topk_workspace_bytes(c.batch, n, c.kv_heads, c.q_heads), shape)
+        aw, _ = ops.workspaces.get("attn", self.device, _lib.lib.sl_sparse_attn_workspace_bytes(c.batch, c.kv_heads, c.q_heads), shape)
+        a.d_scan_workspace, a.scan_workspace_bytes, a.d_status = sw.data_ptr(), sw.numel(), status.data_ptr()
+        a.d_attn_workspace, a.attn_workspace_bytes = aw.data_ptr(), aw.numel()
+        clocks = stats = None
+        lru = self.lru is not None and self.use_lru
+        if lru:
+            lw = ops._lru_ws(self.lru[0], c.batch, c.kv_heads, self.idx.shape[2], self.device)      # the layers follow one another
+            a.d_lru_workspace, a.lru_workspace_bytes = lw.data_ptr(), lw.numel()
+            clocks = (C.c_int * L)(*[t.step for t in self.lru])
+            stats = (C.c_void_p * L)(*[t.status.data_ptr() for t in self.lru])
+        try:
+            _lib.check(_lib.lib.sl_decode_step_lru(C.byref(a), pos, clocks, stats, ops._stream()))
+        finally:
+            if lru:
+                for t, clock in zip(self.lru, clocks):
+                    t.step = clock
+        fill = c.dtype == torch.bfloat16 and c.q_heads // c.kv_heads <= 16
+        ops.launch_count += (3 if not lru else 4 if fill else 5) * L
+
+    def _step_args(self):
+        """The argument block of sl_decode_step over this session's buffers, without the workspaces, and what it points to."""
+        import ctypes as C
+        from . import _lib
+        c, L = self.cfg, self.cfg.layers
+        arr = lambda ts: (C.c_void_p * L)(*[t.data_ptr() for t in ts])
+
+        def rows(t):                                 # the layers' slices of a [L, ...] tensor
+            base, step = t.data_ptr(), t.stride(0) * t.element_size()
+            return (C.c_void_p * L)(*range(base, base + L * step, step))
+
+        a = _lib.DecodeStepArgs()
+        a.B, a.QH, a.KH, a.layers = c.batch, c.q_heads, c.kv_heads, L
+        a.dtype, a.gqa_layout = ops._dt(self.q_in), c.layout
+        a.sink, a.recent, a.min_remain, a.mask_out = c.sink, c.recent, c.min_remain, c.mask_out
+        a.code_batch_stride = self.codes[0].stride(0)
+        kv = ops._kv_layout(self.k_cache[0])
+        a.kv_batch_stride, a.kv_token_stride, a.kv_head_stride = kv.batch_stride, kv.token_stride, kv.head_stride
+        keep = {"q": rows(self.q_in), "k": rows(self.k_in), "v": rows(self.v_in), "codes": arr(self.codes), "kc": arr(self.k_cache),
+                "vc": arr(self.v_cache), "out": rows(self.out),
+                "hq": (_lib.HashParamsStruct * L)(*[h.struct for h in self.hash_q]),
+                "hk": (_lib.HashParamsStruct * L)(*[h.struct for h in self.hash_k])}
+        a.d_q, a.d_k, a.d_v = keep["q"], keep["k"], keep["v"]
+        a.hash_q, a.hash_k = keep["hq"], keep["hk"]
+        a.d_code_cache, a.d_k_cache, a.d_v_cache, a.d_out = keep["codes"], keep["kc"], keep["vc"], keep["out"]
+        a.d_cos, a.d_sin = self.cos.data_ptr(), self.sin.data_ptr()
+        a.d_q_rot, a.d_q_codes = self.q_rot.data_ptr(), self.q_codes.data_ptr()
+        a.d_idx, a.idx_capacity, a.d_cnt = self.idx.data_ptr(), self.idx.shape[2], self.cnt.data_ptr()
+        if self.lru is not None and self.use_lru:   # stage 3: the attended keys are made resident, attention reads the resident buffers
+            keep["lru"] = (_lib.LruLayer * L)()
+            for l, t in enumerate(self.lru):
+                keep["lru"][l].d_k_resident, keep["lru"][l].d_v_resident = t.k.data_ptr(), t.v.data_ptr()
+                keep["lru"][l].d_tok2slot, keep["lru"][l].d_slot2tok = t.tok2slot.data_ptr(), t.slot2tok.data_ptr()
+                keep["lru"][l].d_last_used, keep["lru"][l].d_stats = t.last_used.data_ptr(), t.stats.data_ptr()
+            a.lru = keep["lru"]
+            a.lru_slots, a.lru_n_max = c.lru_slots, c.capacity
+            res = ops._kv_layout(self.lru[0].k)
+            a.lru_batch_stride, a.lru_token_stride, a.lru_head_stride = res.batch_stride, res.token_stride, res.head_stride
+            a.d_slots = self.slots.data_ptr()
+        return a, keep
+
+    def _native_args(self):
         from . import _lib
         c = self.cfg
         assert not c.fix_layers
         if getattr(self, "_native", None) is None:
             self._native = {}
         if self.use_lru not in self._native:
-            L = c.layers
-            arr = lambda ts: (C.c_void_p * L)(*[t.data_ptr() for t in ts])
-            a = _lib.DecodeStepArgs()
-            a.B, a.QH, a.KH, a.layers = c.batch, c.q_heads, c.kv_heads, L
-            a.dtype, a.gqa_layout = ops._dt(self.q_in), c.layout
-            a.sink, a.recent, a.min_remain, a.mask_out = c.sink, c.recent, c.min_remain, c.mask_out
-            a.code_batch_stride = self.codes[0].stride(0)
-            kv = ops._kv_layout(self.k_cache[0])
-            a.kv_batch_stride, a.kv_token_stride, a.kv_head_stride = kv.batch_stride, kv.token_stride, kv.head_stride
-            keep = {"q": arr([self.q_in[l] for l in range(L)]), "k": arr([self.k_in[l] for l in range(L)]),
-                    "v": arr([self.v_in[l] for l in range(L)]), "codes": arr(self.codes), "kc": arr(self.k_cache),
-                    "vc": arr(self.v_cache), "out": arr([self.out[l] for l in range(L)]),
-                    "hq": (_lib.HashParamsStruct * L)(*[h.struct for h in self.hash_q]),
-                    "hk": (_lib.HashParamsStruct * L)(*[h.struct for h in self.hash_k])}
-            a.d_q, a.d_k, a.d_v = keep["q"], keep["k"], keep["v"]
-            a.hash_q, a.hash_k = keep["hq"], keep["hk"]
-            a.d_code_cache, a.d_k_cache, a.d_v_cache, a.d_out = keep["codes"], keep["kc"], keep["vc"], keep["out"]
-            a.d_cos, a.d_sin = self.cos.data_ptr(), self.sin.data_ptr()
-            a.d_q_rot, a.d_q_codes = self.q_rot.data_ptr(), self.q_codes.data_ptr()
-            a.d_idx, a.idx_capacity, a.d_cnt = self.idx.data_ptr(), self.idx.shape[2], self.cnt.data_ptr()
+            a, keep = self._step_args()
             shape = (c.batch, c.kv_heads, c.q_heads)
             sw, status = ops.workspaces.get("scan", self.device, _lib.lib.sl_scan_topk_workspace_bytes(
                 c.batch, c.capacity, c.kv_heads, c.q_heads), shape)
@@ -191,17 +268,7 @@ class DecodeSession:
             a.d_scan_workspace, a.scan_workspace_bytes = sw.data_ptr(), sw.numel()
             a.d_attn_workspace, a.attn_workspace_bytes = aw.data_ptr(), aw.numel()
             a.d_status = status.data_ptr()
-            if self.lru is not None and self.use_lru:   # stage 3: the attended keys are made resident, attention reads the resident buffers
-                keep["lru"] = (_lib.LruLayer * L)()
-                for l, t in enumerate(self.lru):
-                    keep["lru"][l].d_k_resident, keep["lru"][l].d_v_resident = t.k.data_ptr(), t.v.data_ptr()
-                    keep["lru"][l].d_tok2slot, keep["lru"][l].d_slot2tok = t.tok2slot.data_ptr(), t.slot2tok.data_ptr()
-                    keep["lru"][l].d_last_used, keep["lru"][l].d_stats = t.last_used.data_ptr(), t.stats.data_ptr()
-                a.lru = keep["lru"]
-                a.lru_slots, a.lru_n_max = c.lru_slots, c.capacity
-                res = ops._kv_layout(self.lru[0].k)
-                a.lru_batch_stride, a.lru_token_stride, a.lru_head_stride = res.batch_stride, res.token_stride, res.head_stride
-                a.d_slots = self.slots.data_ptr()
+            if self.lru is not None and self.use_lru:
                 need = _lib.lib.sl_lru_workspace_bytes(c.batch, c.kv_heads, self.idx.shape[2])
                 keep["lru_ws"] = torch.zeros(need, dtype=torch.uint8, device=self.device)
                 a.d_lru_workspace, a.lru_workspace_bytes = keep["lru_ws"].data_ptr(), need

@@ -1,0 +1,82 @@
+"""The decode step in one library call against the calls it stands for, and the attention without an index list."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _hash(heads, gen, dtype):
+    from spotlight_b200 import ops
+    return ops.HashParams([(torch.randn((heads, 128, 128), generator=gen, device="cuda") * 0.05).to(dtype)])
+
+
+def _session(seed, batch, qh, kh, layers, n, dtype, lru_slots=0, fused=True, mask_out=0.9):
+    from spotlight_b200.session import DecodeSession, SessionConfig
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    hq, hk = [_hash(qh, gen, dtype) for _ in range(layers)], [_hash(kh, gen, dtype) for _ in range(layers)]
+    s = DecodeSession(SessionConfig(batch, qh, kh, layers, n + 8, dtype, mask_out, lru_slots=lru_slots, fused_kv=fused), hq, hk)
+    for l in range(layers):
+        s.load_context(l, *(torch.randn((batch, n, kh, 128), generator=gen, device="cuda").to(dtype) for _ in range(2)))
+    return s, gen
+
+
+@pytest.mark.parametrize("batch,qh,kh,layers,n,dtype,lru_slots,fused", [
+    (1, 8, 8, 1, 700, torch.float32, 0, True), (2, 8, 2, 3, 3000, torch.bfloat16, 0, False), (1, 16, 4, 2, 3000, torch.bfloat16, 800, True),
+    (2, 4, 4, 2, 900, torch.float32, 400, True), (1, 8, 8, 2, 900, torch.float16, 0, True)])
+def test_step_is_the_layer_steps(batch, qh, kh, layers, n, dtype, lru_slots, fused):
+    a, gen = _session(5, batch, qh, kh, layers, n, dtype, lru_slots, fused)
+    b, _ = _session(5, batch, qh, kh, layers, n, dtype, lru_slots, fused)
+    for t in range(3):
+        for x, h in (("q_in", qh), ("k_in", kh), ("v_in", kh)):
+            value = torch.randn((layers, batch, h, 128), generator=gen, device="cuda").to(dtype)
+            getattr(a, x).copy_(value)
+            getattr(b, x).copy_(value)
+        for s in (a, b):
+            s.set_position(n + t, 10000.0)
+        assert a._one_call(n + t)
+        a.step(n + t)
+        for l in range(layers):
+            b.layer_step(l, n + t)
+        assert torch.equal(a.out, b.out)
+        for l in range(layers):
+            assert torch.equal(a.k_cache[l][:, : n + t + 1], b.k_cache[l][:, : n + t + 1])
+            assert torch.equal(a.codes[l].view(torch.int32)[:, : n + t + 1], b.codes[l].view(torch.int32)[:, : n + t + 1])
+            if lru_slots:
+                assert a.lru[l].step == b.lru[l].step == t + 1
+                for x in ("tok2slot", "slot2tok", "last_used", "stats", "status"):
+                    assert torch.equal(getattr(a.lru[l], x), getattr(b.lru[l], x)), x
+
+
+def test_step_takes_the_layer_steps_where_one_call_does_not_serve():
+    s, _ = _session(6, 1, 4, 4, 2, 300, torch.bfloat16)
+    assert s._one_call(300) and not s._one_call(308) and not s._one_call(-1)
+    with pytest.raises(AssertionError, match="full"):
+        s.step(308)
+    s.k_cache[1], s.v_cache[1] = s.k_cache[1].contiguous(), s.v_cache[1].contiguous()      # another geometry than layer 0
+    assert not s._one_call(300)
+    s.step(300)
+    s.layer_step = lambda *a: None                               # a caller's own layer loop
+    assert not s._one_call(300)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
+@pytest.mark.parametrize("B,n,QH,KH", [(1, 1, 8, 8), (1, 16, 8, 2), (2, 17, 4, 4), (1, 1000, 32, 8), (3, 4097, 10, 2), (1, 20001, 7, 1), (2, 500, 4, 1)])
+def test_dense_attention_is_the_attention_over_a_list_of_all_keys(B, n, QH, KH, dtype):
+    from spotlight_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    q = torch.randn((B, QH, 128), generator=gen, device="cuda").to(dtype)
+    kv = torch.randn((B, n + 5, KH, 2, 128), generator=gen, device="cuda").to(dtype)
+    idx = torch.arange(n, dtype=torch.int32, device="cuda").expand(B, KH, n).contiguous()
+    cnt = torch.full((B, KH), n, dtype=torch.int32, device="cuda")
+    got = ops.dense_attn_decode(q, kv[:, :, :, 0], kv[:, :, :, 1], n)
+    assert torch.equal(got, ops.sparse_attn_decode(q, kv[:, :, :, 0], kv[:, :, :, 1], idx, cnt))
+
+
+def test_the_hooks_state_names_the_keys_of_a_dense_layer_when_asked():
+    from spotlight_b200.modifiers.spotlight_generation import LayerState
+    st = LayerState(2, 3, 20, torch.bfloat16, "cuda")
+    assert st.last_idx is None and st.last_cnt is None
+    st._last = 7
+    assert torch.equal(st.last_idx, torch.arange(7, dtype=torch.int32, device="cuda").expand(2, 3, 7)) and st.last_cnt.tolist() == [[7] * 3] * 2
+    st.last_cnt = None
+    assert st.last_cnt is None and st.last_idx.shape == (2, 3, 7)
