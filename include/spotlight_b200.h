@@ -412,6 +412,9 @@ int sl_sparse_attn_decode_fill(const void* d_q, void* d_k_resident, void* d_v_re
 int sl_gather_rows(const void* d_cache, int64_t batch_stride, int elem_bytes,
                    const int32_t* d_idx, int idx_capacity, int B, int KH, int budget,
                    void* d_out, void* stream);
+/* The same rows of two caches of one geometry (K and V) in one launch. */
+int sl_gather_rows2(const void* d_cache, const void* d_cache2, int64_t batch_stride, int elem_bytes, const int32_t* d_idx,
+                    int idx_capacity, int B, int KH, int budget, void* d_out, void* d_out2, void* stream);
 
 /* One decode token through all layers, with the layer loop in native code: per layer
  * sl_decode_prepare (token `pos` appended) -> sl_scan_topk over keys 0..pos with the reference's

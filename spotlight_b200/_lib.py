@@ -106,6 +106,7 @@ SIGNATURES = {
     "sl_lru_workspace_bytes": (_Z, [_I, _I, _I]),
     "sl_lru_update_ex": (_I, [_P, _I, _P, _I, _I, _P, _P, _KV, _I, _P, _P, _KV, _I, _P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _Z, _P]),
     "sl_gather_rows": (_I, [_P, _L, _I, _P, _I, _I, _I, _I, _P, _P]),
+    "sl_gather_rows2": (_I, [_P, _P, _L, _I, _P, _I, _I, _I, _I, _P, _P, _P]),
     "sl_decode_step": (_I, [C.POINTER(DecodeStepArgs), _L, _P]),
     "sl_decode_step_lru": (_I, [C.POINTER(DecodeStepArgs), _L, C.POINTER(_I), _PP, _P]),
     "sl_decode_step_dev": (_I, [C.POINTER(DecodeStepArgs), C.POINTER(DecodeDev), _P]),

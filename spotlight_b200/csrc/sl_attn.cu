@@ -236,19 +236,34 @@ __global__ void __launch_bounds__(128) merge_lse_kernel(const float* __restrict_
     out[row * 128 + col] = sl::VT<T>::from_f(L > 0.0f ? O / L : 0.0f);
 }
 
-__global__ void __launch_bounds__(256) gather_rows_kernel(const unsigned char* __restrict__ cache, long long bstride_bytes,
-                                                          int row_bytes, const int* __restrict__ idx, int cap, int KH,
-                                                          int budget, unsigned char* __restrict__ out) {
-    // one warp-group of row_bytes/16 lanes copies one row
-    const int lanes = row_bytes / 16;
-    const int rows_per_block = 256 / lanes;
-    const int b = blockIdx.y;
-    const long long r = (long long)blockIdx.x * rows_per_block + threadIdx.x / lanes;   // r = j*KH + h
-    if (threadIdx.x / lanes >= rows_per_block || r >= (long long)budget * KH) return;
-    const int j = (int)(r / KH), h = (int)(r % KH);
-    const long long tok = idx[((long long)b * KH + h) * cap + j];
-    const uint4 v = sl::ld_gather_v4(cache + b * bstride_bytes + (tok * KH + h) * row_bytes + (threadIdx.x % lanes) * 16);
-    *reinterpret_cast<uint4*>(out + (((long long)b * budget + j) * KH + h) * row_bytes + (threadIdx.x % lanes) * 16) = v;
+// One or two caches (K and V) of one geometry, blockIdx.z; a group of row_bytes/16 lanes copies GR rows at a time, so that a
+// thread has GR 16-byte pieces in flight (one before: 11.4 us per cache of 8 x 2642 x 4 rows; now 13.9 us for both).
+constexpr int GR = 4;
+__global__ void __launch_bounds__(256) gather_rows_kernel(const unsigned char* __restrict__ cache0, const unsigned char* __restrict__ cache1,
+                                                          long long bstride_bytes, int row_bytes, const int* __restrict__ idx, int cap, int KH,
+                                                          int budget, unsigned char* __restrict__ out0, unsigned char* __restrict__ out1) {
+    const int lanes = row_bytes / 16, groups = 256 / lanes;              // 16 (2-byte types) or 32 (4-byte types)
+    const int b = blockIdx.y, grp = threadIdx.x / lanes, c = (threadIdx.x % lanes) * 16;
+    const unsigned char* cache = blockIdx.z ? cache1 : cache0;
+    unsigned char* out = (blockIdx.z ? out1 : out0) + (long long)b * budget * KH * row_bytes + c;
+    const unsigned rows = (unsigned)budget * (unsigned)KH, r0 = blockIdx.x * (unsigned)(groups * GR) + (unsigned)grp;    // row r = j*KH + h
+    int tok[GR];
+#pragma unroll
+    for (int u = 0; u < GR; ++u) {
+        const unsigned r = r0 + (unsigned)(u * groups);
+        tok[u] = r < rows ? idx[((long long)b * KH + r % (unsigned)KH) * cap + r / (unsigned)KH] : 0;
+    }
+    uint4 v[GR];
+#pragma unroll
+    for (int u = 0; u < GR; ++u) {
+        const unsigned r = r0 + (unsigned)(u * groups);
+        if (r < rows) v[u] = sl::ld_gather_v4(cache + b * bstride_bytes + ((long long)tok[u] * KH + r % (unsigned)KH) * row_bytes + c);
+    }
+#pragma unroll
+    for (int u = 0; u < GR; ++u) {
+        const unsigned r = r0 + (unsigned)(u * groups);
+        if (r < rows) *reinterpret_cast<uint4*>(out + (long long)r * row_bytes) = v[u];
+    }
 }
 
 int pick_splits(int B, int KH, int cap) {
@@ -409,19 +424,25 @@ extern "C" int sl_merge_lse(const float* d_o, const float* d_lse, int R, int64_t
 
 extern "C" int sl_gather_rows(const void* d_cache, int64_t batch_stride, int elem_bytes, const int32_t* d_idx,
                               int idx_capacity, int B, int KH, int budget, void* d_out, void* stream) {
-    SL_REQUIRE(d_cache && d_idx && d_out, SL_EINVAL, "sl_gather_rows: null pointer");
+    return sl_gather_rows2(d_cache, nullptr, batch_stride, elem_bytes, d_idx, idx_capacity, B, KH, budget, d_out, nullptr, stream);
+}
+
+extern "C" int sl_gather_rows2(const void* d_cache, const void* d_cache2, int64_t batch_stride, int elem_bytes, const int32_t* d_idx,
+                               int idx_capacity, int B, int KH, int budget, void* d_out, void* d_out2, void* stream) {
+    SL_REQUIRE(d_cache && d_idx && d_out && (d_cache2 == nullptr) == (d_out2 == nullptr), SL_EINVAL, "sl_gather_rows: null pointer");
     SL_REQUIRE(B > 0 && B <= 65535 && KH > 0 && budget >= 0 && budget <= idx_capacity, SL_ESHAPE, "sl_gather_rows: bad shape");
     SL_REQUIRE(elem_bytes == 2 || elem_bytes == 4, SL_EINVAL, "sl_gather_rows: elem_bytes must be 2 or 4");
-    SL_REQUIRE(sl::aligned16(d_cache) && sl::aligned16(d_out) && (batch_stride * elem_bytes) % 16 == 0, SL_EALIGN,
-               "sl_gather_rows: buffers must be 16-byte aligned");
+    SL_REQUIRE(sl::aligned16(d_cache) && sl::aligned16(d_out) && sl::aligned16(d_cache2) && sl::aligned16(d_out2) && (batch_stride * elem_bytes) % 16 == 0,
+               SL_EALIGN, "sl_gather_rows: buffers must be 16-byte aligned");
     if (budget == 0) return SL_OK;
     const int row_bytes = 128 * elem_bytes;
-    const int rows_per_block = 256 / (row_bytes / 16);
+    const int rows_per_block = GR * (256 / (row_bytes / 16));
     const long long rows = (long long)budget * KH;
-    dim3 grid((unsigned)((rows + rows_per_block - 1) / rows_per_block), (unsigned)B);
+    SL_REQUIRE(rows < (1ll << 31), SL_ESHAPE, "sl_gather_rows: budget * KH exceeds 2^31");
+    dim3 grid((unsigned)((rows + rows_per_block - 1) / rows_per_block), (unsigned)B, d_cache2 ? 2u : 1u);
     gather_rows_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const unsigned char*>(d_cache), batch_stride * elem_bytes, row_bytes, d_idx, idx_capacity, KH, budget,
-        static_cast<unsigned char*>(d_out));
+        static_cast<const unsigned char*>(d_cache), static_cast<const unsigned char*>(d_cache2), batch_stride * elem_bytes, row_bytes, d_idx,
+        idx_capacity, KH, budget, static_cast<unsigned char*>(d_out), static_cast<unsigned char*>(d_out2));
     SL_CUDA_OK(cudaGetLastError());
     return SL_OK;
 }

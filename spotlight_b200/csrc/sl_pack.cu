@@ -76,32 +76,43 @@ __global__ void __launch_bounds__(256) scores_kernel(const uint32_t* __restrict_
     }
 }
 
-// 128-bit codes with the kv heads dividing the block size: every thread keeps one head, scores
-// with the bit-sliced carry-save scorer (P + 2 popcounts per key instead of 4*G) and streams
-// four 16-byte loads at a time.
+// 128-bit codes with the kv heads dividing the warp: every lane keeps one head and scores with the bit-sliced carry-save scorer
+// (P + 2 popcounts per key instead of 4*G). A warp takes tiles of 256 consecutive codes, eight 16-byte loads per lane, the
+// next tile's under the arithmetic of this one; one wave of CTAs, the first loads ahead of the query planes.
+// 8 x 131 072 x 4 codes, groups of 7: 17.3 us (23.6 with single codes strided over the grid, four loads and two waves).
+constexpr int SCORES_CTAS = 2, SCORES_U = 8;
 template <int P>
-__global__ void __launch_bounds__(256) scores_sliced_kernel(const uint32_t* __restrict__ q, const uint4* __restrict__ k,
-                                                            int64_t k_bstride16, int16_t* __restrict__ out, int64_t N,
-                                                            int KH, int G, int layout) {
+__global__ void __launch_bounds__(256, SCORES_CTAS) scores_sliced_kernel(const uint32_t* __restrict__ q, const uint4* __restrict__ k,
+                                                                         int64_t k_bstride16, int16_t* __restrict__ out, int64_t N,
+                                                                         int KH, int G, int layout) {
+    constexpr int U = SCORES_U;
     __shared__ __align__(16) uint32_t planes[32 * 2 * 4 * 4];          // [KH][2][P][4], KH <= 32
     __shared__ __align__(16) int pbase[32 * 4];
-    const int b = blockIdx.y;
-    stage_planes<P>(q + (int64_t)b * KH * G * 4, KH, G, layout, planes, pbase, threadIdx.x >> 5, 8, threadIdx.x & 31);
+    const int b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t total = N * KH, step = (int64_t)gridDim.x * 8 * (32 * U);
+    const uint4* kb = k + (int64_t)b * k_bstride16;
+    int64_t i0 = ((int64_t)blockIdx.x * 8 + warp) * (32 * U) + lane;
+    uint4 c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (i0 + 32 * u < total) c[u] = sl::ld_stream_v4(kb + i0 + 32 * u);
+    stage_planes<P>(q + (int64_t)b * KH * G * 4, KH, G, layout, planes, pbase, warp, 8, lane);
     __syncthreads();
     uint32_t M[P][4], Mp[P][4];
-    const int base = load_planes<P>(planes, pbase, threadIdx.x % KH, M, Mp);
+    const int base = load_planes<P>(planes, pbase, lane % KH, M, Mp);
     const int sh = sliced_shift(G);
-    const int64_t total = N * KH, stride = (int64_t)gridDim.x * 256;
-    const uint4* kb = k + (int64_t)b * k_bstride16;
     int16_t* ob = out + (int64_t)b * total;
-    for (int64_t i0 = (int64_t)blockIdx.x * 256 + threadIdx.x; i0 < total; i0 += 4 * stride) {
-        uint4 c[4];
+#pragma unroll 1
+    for (; i0 < total; i0 += step) {
+        int s[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (i0 + u * stride < total) c[u] = sl::ld_stream_v4(kb + i0 + u * stride);
+        for (int u = 0; u < U; ++u) s[u] = base + (sliced_score<P>(c[u], M, Mp) << sh);
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (i0 + u * stride < total) ob[i0 + u * stride] = (int16_t)(base + (sliced_score<P>(c[u], M, Mp) << sh));
+        for (int u = 0; u < U; ++u)
+            if (i0 + step + 32 * u < total) c[u] = sl::ld_stream_v4(kb + i0 + step + 32 * u);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i0 + 32 * u < total) ob[i0 + 32 * u] = (int16_t)s[u];
     }
 }
 
@@ -168,6 +179,7 @@ extern "C" int sl_hamming_scores(const uint32_t* d_q, const uint32_t* d_k, int64
     if (W == 4 && KH <= 32 && 32 % KH == 0 && sliced_planes(G) > 0) {
         const uint4* k16 = reinterpret_cast<const uint4*>(d_k);
         const int64_t kb16 = k_batch_stride / 4;
+        grid.x = (unsigned)std::max<int64_t>(1, std::min<int64_t>((total + 256 * SCORES_U - 1) / (256 * SCORES_U), (int64_t)sl::sm_count() * SCORES_CTAS / B));
         switch (sliced_planes(G)) {
             case 1: scores_sliced_kernel<1><<<grid, 256, 0, s>>>(d_q, k16, kb16, d_out, N, KH, G, gqa_layout); break;
             case 2: scores_sliced_kernel<2><<<grid, 256, 0, s>>>(d_q, k16, kb16, d_out, N, KH, G, gqa_layout); break;

@@ -79,10 +79,12 @@ struct LeanArgs {
     int R, rank;
     unsigned long long slot_stride, pflags_off;
     int kk;                    // min(k, global number of keys)
+    const unsigned short* given;   // scores [B,N,KH] of the caller, or null: scored from the codes
     unsigned long long* dbg;   // optional [grid][16] phase stamps (profiling builds only)
 };
 
 bool lean_covers(int KH, int G, int ctas_per_b, int chunk, int nwin);
+bool lean_covers_given(int KH, int nbins, int ctas_per_b, int chunk, int nwin);   // the form whose scores the caller brings
 int lean_nc(int nbins);
 size_t lean_plan_smem(LeanArgs& f, int KH, int nbins, int S, int chunk);   // fills the offsets, returns the total
 int launch_lean(const LeanArgs& a, size_t smem, cudaStream_t s);

@@ -671,8 +671,8 @@ WsLayout ws_layout(int B, long long N, int KH, int G, bool with_hist, bool spill
     w.seg_off = off; off = align_up(off + (size_t)B * max_cpb * KH * 16, 256);
     w.score_off = off; if (spill) off = align_up(off + (size_t)B * N * KH * 2, 256);
     w.epoch_off = w.chist2_off = w.pub_off = w.puba_off = w.wsc_off = off;
-    if (with_hist && nbins <= 0) {
-        const int nb = 128 * G + 1;
+    if (with_hist && (nbins <= 0 || slscan::lean_nc(nbins) <= 32 * slscan::LEAN_CPL_MAX)) {
+        const int nb = nbins > 0 ? nbins : 128 * G + 1;
         w.epoch_off = off; off = align_up(off + (size_t)B * 4, 256);
         w.chist2_off = off; off = align_up(off + (size_t)2 * B * KH * slscan::lean_nc(nb) * 4, 256);
         w.pub_off = off; off = align_up(off + (size_t)std::max(B, sl::sm_count()) * KH * slscan::lean_nc(nb) * 16, 256);
@@ -1041,11 +1041,36 @@ extern "C" int sl_topk_from_scores(const int16_t* d_scores, int B, int64_t N, in
         SL_CUDA_OK(cudaMemsetAsync(d_cnt, 0, (size_t)B * KH * 4, s));
         return SL_OK;
     }
-    const Plan p = make_plan_given_scores(B, N, KH, 1, max_score + 1);
     const WsLayout w = ws_layout(B, N, KH, 1, true, false, max_score + 1);
     SL_REQUIRE(workspace_bytes >= w.total, SL_EWORKSPACE, "sl_topk_from_scores: workspace %zu < required %zu",
                workspace_bytes, w.total);
     unsigned char* ws = static_cast<unsigned char*>(d_workspace);
+    const int s_end0 = (int)std::min<int64_t>(sink, N);
+    const int nwin = s_end0 + (int)(N - std::max<int64_t>(s_end0, N - recent));
+    const Plan q = make_plan(B, N, KH, 1, false, max_score + 1);
+    if (g_lean == 1 && q.cooperative && !q.spill && B * q.ctas_per_b <= sl::sm_count() && (reinterpret_cast<uintptr_t>(d_scores) & 1u) == 0 &&
+        sl::aligned16(d_workspace) && slscan::lean_covers_given(KH, q.nbins, q.ctas_per_b, q.chunk, nwin)) {
+        // the one-barrier kernel of the decode step, fed with scores
+        slscan::LeanArgs f = {};
+        f.given = reinterpret_cast<const unsigned short*>(d_scores);
+        f.B = B; f.KH = KH; f.G = 1; f.N = (int)N; f.k_budget = k;
+        f.s_end = s_end0; f.r_start = (int)std::max<int64_t>(s_end0, N - recent);
+        f.idx = d_idx; f.cap = idx_capacity; f.cnt = d_cnt;
+        f.sync = reinterpret_cast<unsigned*>(ws + w.sync_off);
+        f.epoch = reinterpret_cast<unsigned*>(ws + w.epoch_off);
+        f.chist = reinterpret_cast<unsigned*>(ws + w.chist2_off);
+        f.pub = reinterpret_cast<uint4*>(ws + w.pub_off);
+        f.puba = reinterpret_cast<unsigned short*>(ws + w.puba_off);
+        f.wsc = reinterpret_cast<unsigned short*>(ws + w.wsc_off);
+        f.status = d_status;
+        f.ctas_per_b = q.ctas_per_b; f.chunk = q.chunk; f.nbins = q.nbins; f.S = q.S;
+        f.NC = slscan::lean_nc(q.nbins);
+        f.nc_magic = (unsigned)(((1ull << 32) + f.NC - 1) / f.NC);
+        f.rowh = 2 * ((q.chunk >> 1) + ((4 - (q.chunk >> 1)) & 31));
+        const size_t smem = slscan::lean_plan_smem(f, KH, q.nbins, q.S, q.chunk);
+        if (smem <= (size_t)SMEM_BUDGET + 24 * 1024) return slscan::launch_lean(f, smem, s);
+    }
+    const Plan p = make_plan_given_scores(B, N, KH, 1, max_score + 1);
     ScanArgs a = {};
     a.B = B; a.KH = KH; a.G = 1; a.N = (int)N;
     a.k_budget = k;

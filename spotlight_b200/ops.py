@@ -764,3 +764,19 @@ def gather_rows(cache: torch.Tensor, idx: torch.Tensor, budget: int, device=None
                              out.data_ptr(), _stream()))
     _count()
     return out
+
+
+def gather_kv(keys: torch.Tensor, vals: torch.Tensor, idx: torch.Tensor, budget: int):
+    """gather_rows of two caches; one launch where they share geometry and device."""
+    if not (keys.is_cuda and vals.is_cuda and keys.shape == vals.shape and keys.stride() == vals.stride() and keys.dtype == vals.dtype
+            and keys.device == vals.device):
+        return gather_rows(keys, idx, budget), gather_rows(vals, idx, budget)
+    B, N, KH, D = keys.shape
+    assert D == 128
+    dev = _cuda(keys, vals, idx)
+    cb = _rows_view(keys, 128)
+    k, v = (torch.empty((B, budget, KH, D), dtype=keys.dtype, device=dev) for _ in range(2))
+    check(lib.sl_gather_rows2(keys.data_ptr(), vals.data_ptr(), cb, keys.element_size(), idx.data_ptr(), idx.shape[2], B, KH, budget,
+                              k.data_ptr(), v.data_ptr(), _stream()))
+    _count()
+    return k, v

@@ -1,0 +1,66 @@
+"""Top-k over given scores on the one-barrier kernel against the general kernel and a stable sort, and the two-cache gather."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(scores, k, sink, recent):
+    """Ascending indices of the k best scores (lowest index wins a tie) and the window, per batch row and head."""
+    B, N, KH = scores.shape
+    out = {}
+    for b in range(B):
+        for h in range(KH):
+            top = np.argsort(-scores[b, :, h].astype(np.int64), kind="stable")[: min(k, N)]
+            out[b, h] = np.union1d(np.union1d(top, np.arange(min(sink, N))), np.arange(max(0, N - recent), N))
+    return out
+
+
+# batch rows whose scores do not start on a 16-byte boundary, chunks that end inside a group of eight scores, one head and 32, a
+# single chunk (general kernel), heads that are no power of two (general kernel), windows, ties everywhere, k = 0 and k = N
+@pytest.mark.parametrize("B,N,KH,max_score,k,sink,recent", [
+    (1, 4097, 8, 512, 400, 0, 0), (3, 5003, 1, 128, 500, 4, 64), (8, 9001, 4, 896, 181, 0, 0), (2, 3333, 2, 256, 3333, 0, 0),
+    (2, 2049, 32, 128, 0, 4, 60), (1, 20011, 16, 256, 2000, 0, 90), (1, 100, 8, 512, 10, 0, 0), (2, 6001, 6, 384, 77, 4, 64), (1, 70000, 8, 3, 9999, 0, 0)])
+def test_topk_from_scores(B, N, KH, max_score, k, sink, recent):
+    from spotlight_b200 import _lib, ops
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    mean = max_score / 2
+    s = (mean + max_score ** 0.5 / 2 * torch.randn((B, N, KH), generator=gen, device="cuda")).round().clamp(0, max_score).to(torch.int16)
+    ref = _reference(s.cpu().numpy(), k, sink, recent)
+    got = {}
+    for kernel in (1, 0):
+        ops.configure(_lib.SL_OPT_SCAN_KERNEL, kernel)
+        try:
+            for _ in range(3):                               # the coarse histogram's two buffers take turns
+                idx, cnt = ops.topk_from_scores(s, k, max_score, sink, recent)
+        finally:
+            ops.configure(_lib.SL_OPT_SCAN_KERNEL, 1)
+        got[kernel] = idx.cpu().numpy(), cnt.cpu().numpy()
+    ops.check_status(torch.device("cuda", 0))
+    for idx, cnt in got.values():
+        for (b, h), want in ref.items():
+            assert cnt[b, h] == len(want)
+            np.testing.assert_array_equal(idx[b, h, : cnt[b, h]], want)
+
+
+def test_topk_from_scores_clamps_to_the_given_range():
+    from spotlight_b200 import ops
+    s = torch.randint(0, 100, (2, 3001, 4), device="cuda", dtype=torch.int16)
+    s[0, 17, 2], s[1, 2999, 0] = 3000, -5
+    c = s.clamp(0, 128)
+    for a, b in zip(ops.topk_from_scores(s, 300, 128), ops.topk_from_scores(c, 300, 128)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,N,KH,budget", [(1, 50, 3, 1), (2, 300, 4, 63), (3, 1000, 8, 129), (1, 65, 1, 65)])
+def test_gather_kv(B, N, KH, budget, dtype):
+    from spotlight_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    k, v = (torch.randn((B, N + 7, KH, 128), generator=gen, device="cuda").to(dtype)[:, :N] for _ in range(2))
+    idx = torch.randint(0, N, (B, KH, budget + 2), generator=gen, device="cuda", dtype=torch.int32)
+    at = idx[:, :, :budget].long().transpose(1, 2)[..., None].expand(-1, -1, -1, 128)
+    for got, src in zip(ops.gather_kv(k, v, idx, budget), (k, v)):
+        assert torch.equal(got, src.gather(1, at))
+    assert torch.equal(ops.gather_rows(k, idx, budget), k.gather(1, at))
