@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(MW * 32, 8 / MW) sparse_attn_mma_kernel(const 
         for (int it = 0; it < 8; ++it) {
             const int r = 2 * it + (lane >> 4);
             const int e = __shfl_sync(0xffffffffu, e_own, r);
-            if (e < 0) {
+            if (e < 0 && e != sl::SL_LRU_NO_SLOT) {
                 const long long off = (long long)(-e - 1) * row_stride;
                 *reinterpret_cast<uint4*>(kw + off) = *reinterpret_cast<const uint4*>(sb + swz(r, c));
                 *reinterpret_cast<uint4*>(vw + off) = *reinterpret_cast<const uint4*>(sb + 4096 + swz(r, c));

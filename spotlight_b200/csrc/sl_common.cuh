@@ -53,6 +53,10 @@ int decode_prepare_impl(const void* d_q, const void* d_k, const void* d_v, int d
                         void* d_k_cache, void* d_v_cache, const sl_kv_layout* kv, int64_t pos, const DevPos* dp,
                         void* stream);
 
+// A deferred LRU update that could not give out slots (more attended keys than the table holds; status 3) leaves this instead of
+// -(slot + 1): the attention fetches the key's rows from the backing store and writes them nowhere.
+constexpr int SL_LRU_NO_SLOT = -2147483647 - 1;
+
 // New rows of a layer's cache: where the K rows that are hashed go, and the V rows beside them (strides in elements).
 struct LoadRows {
     void* k_cache; void* v_cache; long long cs_b, cs_tok, cs_h;       // at the first new row

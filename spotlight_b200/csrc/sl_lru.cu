@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(LT) lru_update_kernel(const LruArgs a) {
     for (int i = tid; i < NBIN; i += LT) hist[i] = 0;
     __syncthreads();
     if (n > a.C) {                          // the table cannot hold this step's attended set
+        // no slots to give out: entries the attention that follows may read all the same (a miss nobody fills, or any slot)
+        for (int q = part * LT + tid; q < n && a.phase != 2; q += a.parts * LT) out[q] = (a.deferred || a.phase == 1) ? (a.phase == 1 ? -1 : sl::SL_LRU_NO_SLOT) : 0;
         if (tid == 0 && part == 0) {
             if (a.status) atomicExch(a.status, 3);
             if (a.g_m) a.g_m[bh] = 0;
@@ -410,6 +412,7 @@ __global__ void __launch_bounds__(LT) lru_update_multi_kernel(const LruArgs a) {
     if (part == 0 && tid >= 1 && tid <= 3) bar[tid] = 0u;           // the counters of B1..B3: nobody is near them before B0
     __syncthreads();
     if (n > a.C) {                          // the table cannot hold this step's attended set (every CTA of the pair sees it)
+        for (int q = part * LT + tid; q < n; q += P * LT) out[q] = a.deferred ? sl::SL_LRU_NO_SLOT : 0;       // entries the attention may read
         if (tid == 0 && part == 0) {
             if (a.status) atomicExch(a.status, 3);
             if (a.g_m) a.g_m[bh] = 0;

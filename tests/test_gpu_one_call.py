@@ -80,3 +80,25 @@ def test_the_hooks_state_names_the_keys_of_a_dense_layer_when_asked():
     assert torch.equal(st.last_idx, torch.arange(7, dtype=torch.int32, device="cuda").expand(2, 3, 7)) and st.last_cnt.tolist() == [[7] * 3] * 2
     st.last_cnt = None
     assert st.last_cnt is None and st.last_idx.shape == (2, 3, 7)
+
+
+@pytest.mark.parametrize("dtype,lru_slots", [(torch.bfloat16, 100), (torch.float32, 100), (torch.bfloat16, 2100)])
+def test_an_overfull_lru_table_raises_its_status_and_the_attention_stays_in_bounds(dtype, lru_slots):
+    """More attended keys than slots: the update gives out none, and the list it leaves is one the attention can read. In bf16
+    (the attention fetches what is missing itself) the step's output is the one without the table."""
+    from spotlight_b200 import ops
+    n = 20 * lru_slots // 9                                       # half of it attended: 1.1 times the slots, in one CTA and in several
+    s, gen = _session(7, 1, 4, 4, 2, n, dtype, lru_slots=lru_slots, mask_out=0.5)
+    for x in ("q_in", "k_in", "v_in"):
+        getattr(s, x).copy_(torch.randn(getattr(s, x).shape, generator=gen, device="cuda"))
+    s.set_position(n, 10000.0)
+    s.step(n)
+    torch.cuda.synchronize()
+    assert [int(t.status) for t in s.lru] == [3, 3]
+    assert all(int(t.slot2tok.max()) == -1 and not t.k.any() for t in s.lru) or dtype == torch.float32
+    ops.check_status(torch.device("cuda", 0))
+    out = s.out.clone()
+    s.use_lru = False
+    s.step(n)
+    if dtype == torch.bfloat16:
+        assert torch.equal(s.out, out)
