@@ -43,8 +43,7 @@ struct LruArgs {
     int2* g_pairs;                         // [B*KH][cap] {key, slot} of the misses, copied by lru_copy_kernel
     int* g_m;                              // [B*KH] number of misses of the step
     // the update spread over the CTAs of a (b, kv head) pair (lru_update_multi_kernel)
-    unsigned* g_hist;                      // [B*KH][NBIN] ages of the pair's slots, all parts (left zeroed)
-    int2* g_cnt;                           // [B*KH][parts] {older than tau, of age tau} in each part's slot range
+    unsigned* g_hist;                      // [B*KH][parts][NBIN] ages of the slots of each part's range
     int* g_pm;                             // [B*KH][parts] misses in each part's slice of the list
     int* g_vict;                           // [B*KH][cap] slot taken by the r-th miss
     unsigned* g_bar;                       // [B*KH][8] barrier counters of the pair
@@ -80,6 +79,41 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* wsum, int& total
     return before + inc - v;
 }
 
+// Oldest first: {the largest age with a cumulative count >= m, how many slots of exactly that age are taken}. Warp w sums
+// the bins [32 w, 32 w + 32), every warp finds the group the threshold lies in from the 32 sums and the bin inside it from
+// the group's counts, a bin per lane (one warp walking runs of 33 bins took 3 700 clocks). The bin beyond 32 x 32 (free
+// slots) is taken first. All threads return the same; a barrier stands between the caller's counts and their use here.
+__device__ __forceinline__ int2 threshold_age(const unsigned* hist, int* wsum, int m, int* status) {
+    static_assert(NBIN == LT + 1, "a bin per thread and one more");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned s = __reduce_add_sync(0xffffffffu, hist[threadIdx.x]);
+    if (lane == 0) wsum[warp] = (int)s;
+    __syncthreads();
+    const int beyond = (int)hist[LT];
+    int2 out = make_int2(LT, m);
+    if (beyond < m) {
+        auto suffix = [&](int v) {                   // sum over the lanes from this one up
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int o = __shfl_down_sync(0xffffffffu, v, d);
+                if (lane + d < 32) v += o;
+            }
+            return v;
+        };
+        const int g = wsum[lane], sg = suffix(g) + beyond;
+        const unsigned ball = __ballot_sync(0xffffffffu, sg >= m);
+        if (ball == 0u && threadIdx.x == 0 && status) atomicExch(status, 4);      // table state is inconsistent
+        const int L = ball ? 31 - __clz(ball) : 0;                                // a consistent table always has n - hits evictable slots
+        const int above = __shfl_sync(0xffffffffu, sg - g, L);
+        const int v = (int)hist[L * 32 + lane], sv = suffix(v) + above;
+        const unsigned ball2 = __ballot_sync(0xffffffffu, sv >= m);
+        const int l2 = ball2 ? 31 - __clz(ball2) : 0;
+        out = make_int2(L * 32 + l2, m - (ball2 ? __shfl_sync(0xffffffffu, sv - v, l2) : 0));
+    }
+    __syncthreads();                                 // wsum is used again
+    return out;
+}
+
 // Ranks come from bitmaps, not from ordered loops: a flag per slot (or list entry) is packed into
 // 32-bit words by warp ballots, one block scan over the words' popcounts gives every word its
 // prefix, and every element finds its own rank with one more popcount. The kernel has a fixed,
@@ -98,7 +132,7 @@ __global__ void __launch_bounds__(LT) lru_update_kernel(const LruArgs a) {
     unsigned short* age16 = reinterpret_cast<unsigned short*>(p_miss + nw);   // [C]
     __shared__ unsigned hist[NBIN];
     __shared__ int wsum[LW];
-    __shared__ int s_hits, s_tau, s_r;
+    __shared__ int s_hits;
 
     const int h = blockIdx.x, b = blockIdx.y, part = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long bh = (long long)b * a.KH + h;
@@ -211,36 +245,8 @@ __global__ void __launch_bounds__(LT) lru_update_kernel(const LruArgs a) {
         }
     }
     __syncthreads();
-    if (tid < 32) {                         // oldest first: largest age with a cumulative count >= m
-        int tau = NBIN, r = 0;
-        const int BW = (NBIN + 31) >> 5;
-        const int blo = lane * BW, bhi = min(NBIN, blo + BW);
-        unsigned bs = 0;
-        for (int i = blo; i < bhi; ++i) bs += hist[i];
-        unsigned suf = bs;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned v = __shfl_down_sync(0xffffffffu, suf, d);
-            if (lane + d < 32) suf += v;
-        }
-        const unsigned ball = __ballot_sync(0xffffffffu, suf >= (unsigned)m);
-        if (ball == 0u && lane == 0 && a.status) atomicExch(a.status, 4);   // table state is inconsistent
-        const int L = ball ? 31 - __clz(ball) : 0;   // a consistent table always has n - hits evictable slots
-        int tau_l = 0, gt_l = 0;
-        if (lane == L) {
-            unsigned cum = suf - bs;
-            for (int i = bhi - 1; i >= blo; --i) {
-                const unsigned v = hist[i];
-                if (cum + v >= (unsigned)m) { tau_l = i; gt_l = (int)cum; break; }
-                cum += v;
-            }
-        }
-        tau = __shfl_sync(0xffffffffu, tau_l, L);
-        r = m - __shfl_sync(0xffffffffu, gt_l, L);
-        if (lane == 0) { s_tau = tau; s_r = r; }
-    }
-    __syncthreads();
-    const int tau = s_tau, r = s_r;
+    const int2 tr = threshold_age(hist, wsum, m, a.status);
+    const int tau = tr.x, r = tr.y;
 
     // ---- victim bitmaps: every slot older than tau, and the slots of age tau (the first r are taken)
 #pragma unroll 4
@@ -371,10 +377,13 @@ __global__ void __launch_bounds__(LT) lru_update_kernel(const LruArgs a) {
 }
 
 // The same update with EVERY CTA of a (b, kv head) pair working all the way through: a CTA owns a slice of the index list
-// and a range of the slots; what one CTA needs from the others crosses global memory behind four barriers of the pair
+// and a range of the slots; what one CTA needs from the others crosses global memory behind three barriers of the pair
 // (bounded spins; the launch is cooperative, so the CTAs of a pair are resident together):
-//   probe own slice | B0 | ages of own slots -> shared histogram | B1 | threshold age (every CTA for itself), victim bitmaps of own
-//   slots, their counts | B2 | victims of own slots at their global ranks | B3 | own slice's misses take their victims
+//   probe own slice | B0 | ages of own slots -> own histogram, published | B1 | sum of the histograms (and of those of the ranges
+//   before this one): threshold age and the ranks of the own victims, every CTA for itself; victims at their global ranks |
+//   B2 | own slice's misses take their victims
+// One shared histogram with atomics needed another barrier for the ranges' counts: 30 000 clocks for 13 172 entries with 2 192 misses
+// over 18 CTAs per pair, 36 900 before (with the threshold found by a single warp).
 // Same policy, same tables and slots afterwards as lru_update_kernel.
 __global__ void __launch_bounds__(LT) lru_update_multi_kernel(const LruArgs a) {
     extern __shared__ int smem_i[];
@@ -390,7 +399,8 @@ __global__ void __launch_bounds__(LT) lru_update_multi_kernel(const LruArgs a) {
     unsigned short* age16 = reinterpret_cast<unsigned short*>(p_miss + wpp);   // [cwpp * 32]
     __shared__ unsigned hist[NBIN];
     __shared__ int wsum[LW];
-    __shared__ int s_hits, s_tau, s_r, s_gb, s_eb, s_mb;
+    __shared__ unsigned phist[NBIN];
+    __shared__ int s_hits, s_gb, s_mb;
 
     const int h = blockIdx.x, b = blockIdx.y, part = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long bh = (long long)b * a.KH + h;
@@ -409,7 +419,7 @@ __global__ void __launch_bounds__(LT) lru_update_multi_kernel(const LruArgs a) {
 
     if (tid == 0) s_hits = 0;
     for (int i = tid; i < NBIN; i += LT) hist[i] = 0;
-    if (part == 0 && tid >= 1 && tid <= 3) bar[tid] = 0u;           // the counters of B1..B3: nobody is near them before B0
+    if (part == 0 && (tid == 1 || tid == 2)) bar[tid] = 0u;         // the counters of B1 and B2: nobody is near them before B0
     __syncthreads();
     if (n > a.C) {                          // the table cannot hold this step's attended set (every CTA of the pair sees it)
         for (int q = part * LT + tid; q < n; q += P * LT) out[q] = a.deferred ? sl::SL_LRU_NO_SLOT : 0;       // entries the attention may read
@@ -495,42 +505,46 @@ __global__ void __launch_bounds__(LT) lru_update_multi_kernel(const LruArgs a) {
         }
     }
     __syncthreads();
-    unsigned* gh = a.g_hist + bh * NBIN;
-    for (int i = tid; i < NBIN; i += LT)
-        if (hist[i]) atomicAdd(gh + i, hist[i]);
-    sl::grid_barrier(bar + 1, (unsigned)P, a.status);               // B1: the histogram is complete
-    for (int i = tid; i < NBIN; i += LT) hist[i] = __ldcg(gh + i);
-    __syncthreads();
-    if (tid < 32) {                         // oldest first: largest age with a cumulative count >= m
-        const int BW = (NBIN + 31) >> 5;
-        const int blo = lane * BW, bhi = min(NBIN, blo + BW);
-        unsigned bs = 0;
-        for (int i = blo; i < bhi; ++i) bs += hist[i];
-        unsigned suf = bs;
+    unsigned* gh = a.g_hist + bh * P * NBIN;                        // [P][NBIN]: every part's counts
+    gh[part * NBIN + tid] = hist[tid];
+    if (tid == LT - 1) gh[part * NBIN + LT] = hist[LT];
+    sl::grid_barrier(bar + 1, (unsigned)P, a.status);               // B1: the counts of all parts are there
+    {
+        // a bin per thread (the last thread has one more): the pair's counts, and those of the slot ranges before this one
+        unsigned tot = 0, pre = 0, tot2 = 0, pre2 = 0;
+#pragma unroll 1
+        for (int q0 = 0; q0 < P; q0 += 8) {
+            unsigned v[8], w[8];
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned v = __shfl_down_sync(0xffffffffu, suf, d);
-            if (lane + d < 32) suf += v;
-        }
-        const unsigned ball = __ballot_sync(0xffffffffu, suf >= (unsigned)m);
-        if (ball == 0u && lane == 0 && a.status) atomicExch(a.status, 4);   // table state is inconsistent
-        const int L = ball ? 31 - __clz(ball) : 0;
-        int tau_l = 0, gt_l = 0;
-        if (lane == L) {
-            unsigned cum = suf - bs;
-            for (int i = bhi - 1; i >= blo; --i) {
-                const unsigned v = hist[i];
-                if (cum + v >= (unsigned)m) { tau_l = i; gt_l = (int)cum; break; }
-                cum += v;
+            for (int u = 0; u < 8; ++u) {
+                v[u] = q0 + u < P ? __ldcg(gh + (q0 + u) * NBIN + tid) : 0u;
+                w[u] = (q0 + u < P && tid == LT - 1) ? __ldcg(gh + (q0 + u) * NBIN + LT) : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                tot += v[u]; tot2 += w[u];
+                if (q0 + u < part) { pre += v[u]; pre2 += w[u]; }
             }
         }
-        const int tau = __shfl_sync(0xffffffffu, tau_l, L);
-        const int r = m - __shfl_sync(0xffffffffu, gt_l, L);
-        if (lane == 0) { s_tau = tau; s_r = r; }
+        hist[tid] = tot; phist[tid] = pre;
+        if (tid == LT - 1) { hist[LT] = tot2; phist[LT] = pre2; }
+        if (warp == 0) {                     // misses of the slices before this one (published before B0; at most 64 parts)
+            int mb = (lane < part ? __ldcg(a.g_pm + bh * P + lane) : 0) + (lane + 32 < part ? __ldcg(a.g_pm + bh * P + lane + 32) : 0);
+            mb = __reduce_add_sync(0xffffffffu, mb);
+            if (lane == 0) { s_mb = mb; s_gb = 0; }
+        }
     }
     __syncthreads();
-    const int tau = s_tau, r = s_r;
-    // ---- victim bitmaps of the own slots and their counts
+    const int2 tr = threshold_age(hist, wsum, m, a.status);
+    const int tau = tr.x, r = tr.y;
+    {                                        // slots of the ranges before this one that are older than the threshold age, or of it
+        unsigned older = tid > tau ? phist[tid] : 0u;
+        if (tid == LT - 1 && LT > tau) older += phist[LT];
+        older = __reduce_add_sync(0xffffffffu, older);
+        if (lane == 0 && older) atomicAdd(&s_gb, (int)older);
+    }
+    const int s_eb = (int)phist[tau];
+    // ---- victim bitmaps of the own slots and their prefixes
 #pragma unroll 4
     for (int w = cw0 + warp; w < cw1; w += LW) {
         const int s = w * 32 + lane;
@@ -557,20 +571,7 @@ __global__ void __launch_bounds__(LT) lru_update_multi_kernel(const LruArgs a) {
                 pg += __popc(m_gt[w]); pe += __popc(m_eq[w]);
             }
         }
-        if (tid == 0) a.g_cnt[bh * P + part] = make_int2(tg, te);
     }
-    sl::grid_barrier(bar + 2, (unsigned)P, a.status);               // B2: every range's counts are there
-    if (tid == 0) {                          // the ranges before this one, the slices before this one
-        int gb = 0, eb = 0, mb = 0;
-        for (int q = 0; q < part; ++q) {
-            const int2 c = __ldcg(a.g_cnt + bh * P + q);
-            gb += c.x; eb += c.y;
-            mb += __ldcg(a.g_pm + bh * P + q);
-        }
-        s_gb = gb; s_eb = eb; s_mb = mb;
-    }
-    // the pair's histogram is read by everybody by now: this CTA's share of it goes back to zero for the next call
-    for (int i = part * LT + tid; i < NBIN; i += P * LT) gh[i] = 0u;
     __syncthreads();
     int* vict = a.g_vict + bh * a.cap;
 #pragma unroll 4
@@ -580,7 +581,7 @@ __global__ void __launch_bounds__(LT) lru_update_multi_kernel(const LruArgs a) {
         const bool isg = (g >> lane) & 1u, ise = (e >> lane) & 1u;
         if (isg || (ise && eb < r)) vict[gb + min(eb, r)] = (cw0 + w) * 32 + lane;
     }
-    sl::grid_barrier(bar + 3, (unsigned)P, a.status);               // B3: the victims stand at their ranks
+    sl::grid_barrier(bar + 2, (unsigned)P, a.status);               // B2: the victims stand at their ranks
     // ---- the own slice's misses, in list order, take the victims in that order
     int2* pairs = (a.g_pairs && !a.deferred) ? a.g_pairs + bh * a.cap : nullptr;
     for (int wq = warp; wq < w1 - w0; wq += 4 * LW) {
@@ -722,9 +723,8 @@ int lru_launch(const int32_t* d_idx, int idx_capacity, const int32_t* d_cnt, int
         // behind the pairs: what the CTAs of a pair exchange when all of them work through the update
         const size_t bh = (size_t)B * KH;
         a.g_hist = reinterpret_cast<unsigned*>(a.g_pairs + bh * idx_capacity);
-        a.g_bar = a.g_hist + ((bh * NBIN + 3) / 4) * 4;
-        a.g_cnt = reinterpret_cast<int2*>(a.g_bar + bh * 8);
-        a.g_pm = reinterpret_cast<int*>(a.g_cnt + bh * 64);
+        a.g_bar = a.g_hist + ((bh * a.parts * NBIN + 3) / 4) * 4;
+        a.g_pm = reinterpret_cast<int*>(a.g_bar + bh * 8);
         a.g_vict = a.g_pm + bh * 64;
     }
     if (g_lru_multi && phase == 0 && d_workspace && a.parts > 1 && B * KH * a.parts <= sl::sm_count()) {
@@ -761,8 +761,8 @@ extern "C" size_t sl_lru_workspace_bytes(int B, int KH, int idx_capacity) {
     const size_t bh = (size_t)B * KH;
     return ((((size_t)B * KH * 2 + 63) / 64) * 64 + (((size_t)B * KH + 63) / 64) * 64 + (((size_t)B * KH * nw + 3) / 4) * 4) * 4 +
            (size_t)B * KH * idx_capacity * 8 +
-           // histogram of ages, barrier counters, per-part counts ({older, ties}, misses; at most 64 parts), victims
-           (((bh * NBIN + 3) / 4) * 4 + bh * 8) * 4 + bh * 64 * 8 + bh * 64 * 4 + bh * (size_t)idx_capacity * 4;
+           // histograms of ages of the parts, barrier counters, misses of the parts (at most 64), victims
+           (((bh * lru_parts(B, KH, idx_capacity) * NBIN + 3) / 4) * 4 + bh * 8) * 4 + bh * 64 * 4 + bh * (size_t)idx_capacity * 4;
 }
 
 extern "C" int sl_lru_update(const int32_t* d_idx, int idx_capacity, const int32_t* d_cnt, int B, int KH,
