@@ -63,6 +63,12 @@ struct LoadRows {
     const void* v; long long vs_b, vs_tok, vs_h;
 };
 
+int check_hash_params(const char* fn, const sl_hash_params* p, int dtype);
+// Code build of many rows on tcgen05 (sl_hash_tc.cu); with `load` the rows are also stored to the K cache and their V rows
+// copied. 1: not a hash or a shape it covers.
+int launch_hash_encode_tc(const void* x, long long xs_b, long long xs_tok, long long xs_h, int B, long long T, int H, const sl_hash_params* hp,
+                          uint32_t* codes, long long cs_b, const LoadRows* load, cudaStream_t s);
+
 // ---- launches ----------------------------------------------------------------------------
 // Kernels of the decode path are launched with programmatic stream serialisation: a kernel may
 // start while its predecessor in the stream drains, does whatever does not depend on it, and
