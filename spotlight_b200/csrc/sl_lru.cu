@@ -382,8 +382,9 @@ __global__ void __launch_bounds__(LT) lru_update_kernel(const LruArgs a) {
 //   probe own slice | B0 | ages of own slots -> own histogram, published | B1 | sum of the histograms (and of those of the ranges
 //   before this one): threshold age and the ranks of the own victims, every CTA for itself; victims at their global ranks |
 //   B2 | own slice's misses take their victims
-// One shared histogram with atomics needed another barrier for the ranges' counts: 30 000 clocks for 13 172 entries with 2 192 misses
-// over 18 CTAs per pair, 36 900 before (with the threshold found by a single warp).
+// One shared histogram with atomics needed another barrier for the ranges' counts (about 3 100 of 36 900 clocks for 13 172 entries
+// with 2 192 misses over 18 CTAs per pair); with that and the threshold by the whole block eight layers of the 128K
+// four-stage step went from 532 to 516 us.
 // Same policy, same tables and slots afterwards as lru_update_kernel.
 __global__ void __launch_bounds__(LT) lru_update_multi_kernel(const LruArgs a) {
     extern __shared__ int smem_i[];
