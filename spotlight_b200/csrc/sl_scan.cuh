@@ -62,7 +62,7 @@ struct LeanArgs {
     unsigned* chist;           // [2][B][KH][NC] coarse histograms (one per launch parity)
     uint4* pub;                // [B][KH][NC][ctas_per_b] every chunk's counts of each coarse bin's 8 scores, 16 bits each
     unsigned short* puba;      // [B][KH][NC][ctas_per_b] every chunk's keys above each coarse bin
-    unsigned nc_magic;         // ceil(2^32 / NC): i / NC == __umulhi(i, nc_magic) for i < 2^16
+    unsigned nc_magic;         // ceil(2^32 / NC): i / NC == __umulhi(i, nc_magic) for i < 2^16 and NC > 1
     unsigned short* wsc;       // [B][KH][LEAN_MAX_WIN] scores of the always-kept keys
     int* status;
     int ctas_per_b, chunk, nbins, S;

@@ -227,7 +227,8 @@ __global__ void __launch_bounds__(NT, 1) scan_lean_kernel(const LeanArgs a) {
         const size_t pbase = (size_t)b * KH * NC * cpb + c;
 #pragma unroll 1
         for (int i = tid; i < KH * NC; i += NT) {
-            const int h = (int)__umulhi((unsigned)i, a.nc_magic), cb = i - h * NC;
+            // given scores may have a single coarse bin (at most 8 scores): its reciprocal, 2^32, does not fit the word
+            const int h = GIVEN && NC == 1 ? i : (int)__umulhi((unsigned)i, a.nc_magic), cb = i - h * NC;
             const uint4* R = reinterpret_cast<const uint4*>(shist + h * nb1 + (cb << LEAN_CWS));
             const bool two = (cb << LEAN_CWS) + 4 < nb1;
             unsigned v[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};

@@ -44,6 +44,37 @@ def test_topk_from_scores(B, N, KH, max_score, k, sink, recent):
             np.testing.assert_array_equal(idx[b, h, : cnt[b, h]], want)
 
 
+# score ranges of one coarse bin of eight scores and the first of two and three, over heads that share a warp's bins
+@pytest.mark.parametrize("KH", [1, 2, 8, 32])
+@pytest.mark.parametrize("max_score", [0, 1, 2, 3, 4, 5, 6, 7, 8, 15, 16])
+def test_topk_from_scores_of_a_small_range(KH, max_score):
+    from spotlight_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(100 * max_score + KH)
+    s = torch.randint(0, max_score + 1, (2, 1501, KH), generator=gen, device="cuda", dtype=torch.int32).to(torch.int16)
+    s[1] = max_score                                         # every key a tie
+    for k, sink, recent in ((150, 0, 0), (700, 4, 60)):
+        ref = _reference(s.cpu().numpy(), k, sink, recent)
+        for _ in range(2):
+            idx, cnt = (x.cpu().numpy() for x in ops.topk_from_scores(s, k, max_score, sink, recent))
+            for (b, h), want in ref.items():
+                assert cnt[b, h] == len(want)
+                np.testing.assert_array_equal(idx[b, h, : cnt[b, h]], want)
+    ops.check_status(torch.device("cuda", 0))
+
+
+@pytest.mark.parametrize("values", [(0,), (0, 1), (0, 5), (7, 7)])
+def test_topk_and_gather_reads_its_range_from_the_scores(values):
+    from spotlight_b200.modifiers.gpu_cache import topk_and_gather
+    gen = torch.Generator(device="cuda").manual_seed(len(values))
+    pick = torch.randint(0, len(values), (2, 900, 8), generator=gen, device="cuda")
+    s = torch.tensor(values, device="cuda", dtype=torch.int16)[pick]
+    k, v = (torch.randn((2, 900, 8, 128), generator=gen, device="cuda").bfloat16() for _ in range(2))
+    at = torch.stack([torch.tensor(np.stack([np.sort(np.argsort(-s[b, :, h].cpu().numpy().astype(np.int64), kind="stable")[:90]) for h in range(8)], 1)) for b in range(2)])
+    at = at.cuda()[..., None].expand(-1, -1, -1, 128)
+    for got, src in zip(topk_and_gather(s, k, v, 90), (k, v)):
+        assert torch.equal(got, src.gather(1, at))
+
+
 def test_topk_from_scores_clamps_to_the_given_range():
     from spotlight_b200 import ops
     s = torch.randint(0, 100, (2, 3001, 4), device="cuda", dtype=torch.int16)
