@@ -259,12 +259,11 @@ def self_attn_forward(self, hidden_states: torch.Tensor, kv_cache: Optional[Laye
     cos, sin = _rope_table(pos + 1, theta, q.dtype, q.device)
     cos, sin = cos[pos], sin[pos]
     k_cache, v_cache = st.k, st.v
-    if hashed and not per_q and type(kw["mask_out"]) in (int, float) and type(kw.get("min_remain", 20)) is int:
+    keep = budget(pos + 1, kw["mask_out"], kw.get("min_remain", 20)) if hashed and not per_q else None
+    if type(keep) is int and keep >= 0:
         n = pos + 1
-        keep = budget(n, kw["mask_out"], kw.get("min_remain", 20))
         o, idx, cnt = ops.decode_layer(q[:, 0], k[:, 0], v[:, 0], self._hash_q_params(), self._hash_k_params(), pos, st.codes, k_cache, v_cache,
-                                       cos, sin, keep, kw["mask_out"], kw.get("min_remain", 20), int(kw.get("sink", 4)),
-                                       int(kw.get("recent", 64)), GQA_BLOCKED)
+                                       cos, sin, keep, int(kw.get("sink", 4)), int(kw.get("recent", 64)), GQA_BLOCKED)
         st.length = n
         st._last = (idx, cnt)
         return self.o_proj(o.view(B, 1, num_heads * head_dim)), st

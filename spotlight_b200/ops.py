@@ -535,12 +535,18 @@ def dense_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     return out
 
 
+def step_budget(a: "_lib.DecodeStepArgs", keep: int, n: int) -> None:
+    """Makes the library's rule max(min(n, min_remain), n - int(n * mask_out)) come out as `keep`, whatever numbers the caller's
+    own mask_out and min_remain are (an integer beyond 32 bits would wrap in the block)."""
+    a.min_remain, a.mask_out = min(keep, n), 1.0
+
+
 def decode_layer(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, hash_q: HashParams, hash_k: HashParams, pos: int, code_cache: torch.Tensor,
-                 k_cache: torch.Tensor, v_cache: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, keep: int, mask_out: float,
-                 min_remain: int, sink: int, recent: int, layout: int = GQA_BLOCKED):
+                 k_cache: torch.Tensor, v_cache: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, keep: int, sink: int, recent: int,
+                 layout: int = GQA_BLOCKED):
     """decode_prepare, scan_topk and sparse_attn_decode of one layer and token in ONE call into the library: q [B,QH,128], k / v
-    [B,KH,128]; row `pos` of the full caches is written, keys 0 .. pos are scanned. `keep` is budget(pos + 1, mask_out, min_remain),
-    which the library evaluates again by the same rule. Returns (out [B,QH,128], idx, cnt)."""
+    [B,KH,128]; row `pos` of the full caches is written, keys 0 .. pos are scanned, `keep` of them selected beside the window.
+    Returns (out [B,QH,128], idx, cnt)."""
     B, QH, D = q.shape
     KH, n = k.shape[1], pos + 1
     assert D == 128
@@ -563,7 +569,8 @@ def decode_layer(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, hash_q: Hash
     P = C.c_void_p * 1
     a = _lib.DecodeStepArgs()
     a.B, a.QH, a.KH, a.layers, a.dtype, a.gqa_layout = B, QH, KH, 1, _dt(q), layout
-    a.sink, a.recent, a.min_remain, a.mask_out = sink, recent, min_remain, mask_out
+    a.sink, a.recent = sink, recent
+    step_budget(a, keep, n)
     a.code_batch_stride = _rows_view(code_cache, 4)
     a.kv_batch_stride, a.kv_token_stride, a.kv_head_stride = kv.batch_stride, kv.token_stride, kv.head_stride
     a.d_q, a.d_k, a.d_v, a.d_out = P(q.data_ptr()), P(k.data_ptr()), P(v.data_ptr()), P(out.data_ptr())

@@ -160,12 +160,15 @@ class DecodeSession:
             self.layer_step(layer, pos, stage)
 
     def _one_call(self, pos: int) -> bool:
-        """Whether sl_decode_step_lru serves `step(pos)`: the position is inside the caches, no dense layers, layer_step is this
-        class's, and the buffers (which a caller may have exchanged) still have one geometry for all layers."""
+        """Whether sl_decode_step_lru serves `step(pos)`: the position is inside the caches, no dense layers, a whole budget, layer_step
+        is this class's, and the buffers (which a caller may have exchanged) still have one geometry for all layers."""
         c = self.cfg
         if c.fix_layers or not 0 <= pos < c.capacity or type(self).layer_step is not DecodeSession.layer_step or "layer_step" in self.__dict__:
             return False
         L, dt = c.layers, self.q_in.dtype
+        k_budget = budget(pos + 1, c.mask_out, c.min_remain)
+        if type(k_budget) is not int or k_budget < 0:
+            return False
         if not (len(self.codes) == len(self.k_cache) == len(self.v_cache) == len(self.hash_q) == len(self.hash_k) == L):
             return False
         ks, cs, kn, cn = self.k_cache[0].stride(), self.codes[0].stride(), self.k_cache[0].shape, self.codes[0].shape
@@ -190,6 +193,7 @@ class DecodeSession:
         c, L, n = self.cfg, self.cfg.layers, pos + 1
         ops._cuda(self.q_in)
         a, keep = self._step_args()                  # from the buffers as they are now
+        ops.step_budget(a, budget(n, c.mask_out, c.min_remain), n)
         shape = (c.batch, c.kv_heads, c.q_heads)
         sw, status = ops.workspaces.get("scan", self.device, _lib.lib.sl_scan_topk_workspace_bytes(c.batch, n, c.kv_heads, c.q_heads), shape)
         aw, _ = ops.workspaces.get("attn", self.device, _lib.lib.sl_sparse_attn_workspace_bytes(c.batch, c.kv_heads, c.q_heads), shape)
@@ -212,7 +216,8 @@ class DecodeSession:
         ops.launch_count += (3 if not lru else 4 if fill else 5) * L
 
     def _step_args(self):
-        """The argument block of sl_decode_step over this session's buffers, without the workspaces, and what it points to."""
+        """The argument block of sl_decode_step over this session's buffers, without the budget and the workspaces, and what it
+        points to."""
         import ctypes as C
         from . import _lib
         c, L = self.cfg, self.cfg.layers
@@ -225,7 +230,7 @@ class DecodeSession:
         a = _lib.DecodeStepArgs()
         a.B, a.QH, a.KH, a.layers = c.batch, c.q_heads, c.kv_heads, L
         a.dtype, a.gqa_layout = ops._dt(self.q_in), c.layout
-        a.sink, a.recent, a.min_remain, a.mask_out = c.sink, c.recent, c.min_remain, c.mask_out
+        a.sink, a.recent = c.sink, c.recent
         a.code_batch_stride = self.codes[0].stride(0)
         kv = ops._kv_layout(self.k_cache[0])
         a.kv_batch_stride, a.kv_token_stride, a.kv_head_stride = kv.batch_stride, kv.token_stride, kv.head_stride
@@ -260,6 +265,7 @@ class DecodeSession:
             self._native = {}
         if self.use_lru not in self._native:
             a, keep = self._step_args()
+            a.min_remain, a.mask_out = min(c.min_remain, c.capacity), c.mask_out     # no context is longer; a larger integer would wrap
             shape = (c.batch, c.kv_heads, c.q_heads)
             sw, status = ops.workspaces.get("scan", self.device, _lib.lib.sl_scan_topk_workspace_bytes(
                 c.batch, c.capacity, c.kv_heads, c.q_heads), shape)

@@ -1,4 +1,8 @@
 """The decode step in one library call against the calls it stands for, and the attention without an index list."""
+import sys
+import types
+
+import numpy as np
 import pytest
 import torch
 
@@ -57,6 +61,59 @@ def test_step_takes_the_layer_steps_where_one_call_does_not_serve():
     s.step(300)
     s.layer_step = lambda *a: None                               # a caller's own layer loop
     assert not s._one_call(300)
+
+
+# what Python's budget rule takes: integers beyond 32 bits ("never prune"), a budget above and below the other term, numbers that
+# are no int, a mask_out that leaves more than every key
+@pytest.mark.parametrize("mask_out,min_remain", [(0.9, sys.maxsize), (0.9, 2 ** 31), (0.9, 2 ** 32 + 5), (0.9, 20.5), (np.float32(0.9), 20), (1, 33), (0, 20),
+                                                 (-0.5, 20), (1.25, 40)])
+def test_step_keeps_pythons_budget(mask_out, min_remain):
+    n = 700
+    a, gen = _session(8, 1, 8, 2, 2, n, torch.bfloat16)
+    b, _ = _session(8, 1, 8, 2, 2, n, torch.bfloat16)
+    for s in (a, b):
+        s.cfg.mask_out, s.cfg.min_remain = mask_out, min_remain
+        s.idx = torch.empty((1, 2, n + 8), dtype=torch.int32, device="cuda")
+        s.set_position(n, 10000.0)
+    for x in ("q_in", "k_in", "v_in"):
+        getattr(a, x).copy_(torch.randn(getattr(a, x).shape, generator=gen, device="cuda"))
+        getattr(b, x).copy_(getattr(a, x))
+    assert a._one_call(n)
+    a.step(n)
+    for l in range(2):
+        b.layer_step(l, n)
+    assert torch.equal(a.cnt, b.cnt) and torch.equal(a.out, b.out)
+    if min_remain >= 2 ** 31:
+        assert a.cnt.tolist() == [[n + 1] * 2]
+        b.step_native(n)
+        assert b.cnt.tolist() == [[n + 1] * 2] and torch.equal(a.out, b.out)
+
+
+def _hook_layer(qh, kh, gen, **draft):
+    """An attention layer as self_attn_forward meets it, its projections given: (layer, a function that sets q, k and v)."""
+    layer = types.SimpleNamespace(config=types.SimpleNamespace(num_attention_heads=qh, num_key_value_heads=kh, hidden_size=qh * 128, rope_theta=10000.0),
+                                  draft_kwargs={"enable": True, "mask_out": 0.9, **draft}, is_fix_layer=False, o_proj=lambda o: o)
+    hq, hk = _hash(qh, gen, torch.bfloat16), _hash(kh, gen, torch.bfloat16)
+    layer._hash_q_params, layer._hash_k_params = lambda: hq, lambda: hk
+
+    def give(q, k, v):
+        layer.q_proj, layer.k_proj, layer.v_proj = lambda h: q, lambda h: k, lambda h: v
+    return layer, give
+
+
+@pytest.mark.parametrize("min_remain,mask_out", [(sys.maxsize, 0.9), (2 ** 31, 0.9), (2 ** 32 + 5, 0.9), (20, np.float32(0.9)), (30, 0.98)])
+def test_hook_keeps_pythons_budget(min_remain, mask_out):
+    from spotlight_b200.modifiers.spotlight_generation import budget, self_attn_forward
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    layer, give = _hook_layer(8, 2, gen, min_remain=min_remain, mask_out=mask_out, sink=0, recent=0)
+    state = None
+    for T in (900, 1, 1):
+        x = [torch.randn((1, T, h * 128), generator=gen, device="cuda").bfloat16() for h in (8, 2, 2)]
+        give(*x)
+        with torch.no_grad():
+            _, state = self_attn_forward(layer, x[0], state)
+    keep = budget(902, mask_out, min_remain)
+    assert state.last_cnt.tolist() == [[keep] * 2] and (min_remain < 2 ** 31 or keep == 902)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
