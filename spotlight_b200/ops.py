@@ -402,14 +402,16 @@ def untraced(*tensors: torch.Tensor) -> bool:
 
 def prefill_covers(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor) -> bool:
     """Whether rope_append + prefill_attention take these tensors: plain bf16 CUDA tensors nobody differentiates or
-    traces, q [B,T,QH,128] and k / v [B,T,KH,128] with QH a multiple of KH (at most 128 times), cache views whose rows
-    are 16-byte aligned and whose batch rows are distinct."""
+    traces, q [B,T,QH,128] and k / v [B,T,KH,128] with QH a multiple of KH (at most 128 times), 16-byte aligned where
+    they are used as they are (contiguous), cache views whose rows are 16-byte aligned and whose batch rows are distinct."""
     ts = (q, k, v, k_cache, v_cache)
     if not untraced(*ts) or any(t.dtype != torch.bfloat16 or not t.is_cuda or t.device != q.device for t in ts):
         return False
     B, T, QH, D = q.shape
     KH = k.shape[2]
     if D != 128 or k.shape != (B, T, KH, 128) or v.shape != k.shape or QH % KH or QH // KH > 128:
+        return False
+    if B > 65535 or KH > 65535 or any(t.data_ptr() % 16 and t.is_contiguous() for t in (q, k, v)):
         return False
     for c in (k_cache, v_cache):
         sb, st, sh, sd = c.stride()

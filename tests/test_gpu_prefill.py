@@ -1,4 +1,6 @@
 """RoPE + append and the causal attention of a prompt (tcgen05) against plain PyTorch, and against the general path."""
+import types
+
 import pytest
 import torch
 
@@ -95,6 +97,29 @@ def test_the_hook_keeps_the_general_path_for_what_autograd_sees():
         assert not ops.prefill_covers(q, k, v, kc, vc)
     two = kv.expand(2, -1, -1, -1, -1)               # batch rows that share memory
     assert not ops.prefill_covers(q.expand(2, -1, -1, -1), k.expand(2, -1, -1, -1), v.expand(2, -1, -1, -1), two[:, :, :, 0], two[:, :, :, 1])
+
+
+def _dense_layer(qh, kh, q, k, v):
+    """A layer that attends to every key, as the hook meets it, with its projections given."""
+    return types.SimpleNamespace(config=types.SimpleNamespace(num_attention_heads=qh, num_key_value_heads=kh, hidden_size=qh * 128, rope_theta=10000.0),
+                                 draft_kwargs={"enable": True}, is_fix_layer=True, q_proj=lambda h: q, k_proj=lambda h: k, v_proj=lambda h: v, o_proj=lambda o: o)
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("which", ["q", "k", "v"])
+def test_a_prompt_takes_projections_that_start_between_16_byte_boundaries(which):
+    from spotlight_b200 import ops
+    from spotlight_b200.modifiers.spotlight_generation import self_attn_forward
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    x = {n: torch.randn((1, 70, h * 128), generator=gen, device="cuda").bfloat16() for n, h in (("q", 8), ("k", 2), ("v", 2))}
+    want, st0 = self_attn_forward(_dense_layer(8, 2, **x), x["q"])
+    x[which] = torch.empty(x[which].numel() + 1, dtype=torch.bfloat16, device="cuda")[1:].view(x[which].shape).copy_(x[which])
+    got, st = self_attn_forward(_dense_layer(8, 2, **x), x["q"])
+    assert (got.float() - want.float()).norm() <= 5e-3 * want.float().norm()              # the general path's own roundings
+    assert torch.equal(st.k[:, :70], st0.k[:, :70]) and torch.equal(st.v[:, :70], st0.v[:, :70])
+    strided = torch.empty((1, 70, 9, 128), dtype=torch.bfloat16, device="cuda")[:, :, 1:]   # not contiguous: copied, the copy is aligned
+    kc, vc = _caches(1, 80, 2, True, gen)
+    assert ops.prefill_covers(strided, *(torch.zeros((1, 70, 2, 128), dtype=torch.bfloat16, device="cuda") for _ in range(2)), kc, vc)
 
 
 def _hash(kind, heads, gen, dtype=torch.bfloat16):
