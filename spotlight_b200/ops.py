@@ -457,12 +457,12 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
 
 
 def load_rows_covers(k: torch.Tensor, v: torch.Tensor, k_rows: torch.Tensor, v_rows: torch.Tensor) -> bool:
-    """Whether load_rows takes sources k / v for the cache rows k_rows / v_rows (all [B,T,KH,128]): one dtype and device, 16-byte
-    aligned rows, no shared memory (the source may be a view of a cache), nothing traced."""
+    """Whether load_rows takes sources k / v for the cache rows k_rows / v_rows (all [B,T,KH,128]): not empty, one dtype and device,
+    16-byte aligned rows, no shared memory (the source may be a view of a cache), nothing traced."""
     ts = (k, v, k_rows, v_rows)
     if not untraced(*ts) or any(t.shape != k_rows.shape or t.dtype != k_rows.dtype or not t.is_cuda or t.device != k_rows.device for t in ts):
         return False
-    if k_rows.dim() != 4 or k_rows.shape[3] != 128 or k_rows.dtype not in (torch.bfloat16, torch.float16, torch.float32):
+    if k_rows.dim() != 4 or k_rows.shape[3] != 128 or k_rows.numel() == 0 or k_rows.shape[0] > 65535 or k_rows.dtype not in (torch.bfloat16, torch.float16, torch.float32):
         return False
     if any(st % (16 // t.element_size()) for t in ts for st in t.stride()[:3]) or any(t.stride(3) != 1 or t.data_ptr() % 16 for t in ts):
         return False
@@ -480,7 +480,7 @@ def load_rows(k: torch.Tensor, v: torch.Tensor, k_rows: torch.Tensor, v_rows: to
     of the keys into codes [B,T,KH,4] (a view of the code cache). See load_rows_covers."""
     B, T, KH, _ = k_rows.shape
     _cuda(k, v, k_rows, v_rows)
-    assert params is None or (params.heads == KH and codes.shape == (B, T, KH, 4) and codes.dtype == torch.uint32)
+    assert params is None or (params.heads == KH and codes.shape == (B, T, KH, 4) and codes.element_size() == 4)
     kl, vl, cl = _kv_layout(k), _kv_layout(v), _kv_layout(k_rows)
     check(lib.sl_load_rows(k.data_ptr(), C.byref(kl), v.data_ptr(), C.byref(vl), _dt(k), B, T, KH, k_rows.data_ptr(), v_rows.data_ptr(),
                            C.byref(cl), params.ref() if params is not None else None, _ptr(codes),

@@ -190,6 +190,30 @@ def test_load_context_keeps_torchs_copy_for_the_rest():
     assert torch.equal(s.k_cache[0][:, 50, 1], s.k_cache[0][:, 50, 0])
 
 
+@pytest.mark.parametrize("B,T", [(0, 20), (2, 0), (65537, 2)])
+def test_load_context_of_nothing_and_of_very_many_batch_rows(B, T):
+    from spotlight_b200.session import DecodeSession, SessionConfig
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    h = [_hash("linear", 1, gen)]
+    s = DecodeSession(SessionConfig(B, 1, 1, 1, max(T, 1)), h, h)
+    k, v = (torch.randn((B, T, 1, 128), generator=gen, device="cuda").bfloat16() for _ in range(2))
+    s.load_context(0, k, v, 0, codes=False)
+    assert torch.equal(s.k_cache[0][:, :T], k) and torch.equal(s.v_cache[0][:, :T], v)
+
+
+def test_load_context_fills_codes_held_as_signed_words():
+    from spotlight_b200.session import DecodeSession, SessionConfig
+    gen = torch.Generator(device="cuda").manual_seed(13)
+    h = [_hash("linear", 8, gen)]
+    s = DecodeSession(SessionConfig(1, 8, 8, 1, 5000), h, h)
+    k, v = (torch.randn((1, 5000, 8, 128), generator=gen, device="cuda").bfloat16() for _ in range(2))
+    s.load_context(0, k, v)
+    want = s.codes[0].view(torch.int32).clone()
+    s.codes[0] = torch.zeros_like(want)
+    s.load_context(0, k, v)
+    assert torch.equal(s.codes[0], want)
+
+
 def test_the_hash_kernels_silu_is_the_accurate_formula_for_every_bf16():
     """Every finite bf16 through the tcgen05 kernel's activation: with an identity first layer, hidden value j of a row is
     silu(x_j); +-identity in the second layer and torch's value (fp32 x / (1 + exp(-x)), rounded once) taken off as the bias
