@@ -15,6 +15,8 @@ from ._lib import GQA_BLOCKED, GQA_INTERLEAVED, check, lib
 _DTYPES = {torch.bfloat16: _lib.SL_BF16, torch.float32: _lib.SL_F32, torch.float16: _lib.SL_F16,
            torch.bool: _lib.SL_BOOL}
 
+_ROW_BYTES = {torch.bfloat16: 2, torch.float16: 2, torch.float32: 4}      # bytes of a value in the caches' types
+
 launch_count = 0     # kernels launched through this module (bench accounting)
 
 
@@ -458,20 +460,25 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
 
 def load_rows_covers(k: torch.Tensor, v: torch.Tensor, k_rows: torch.Tensor, v_rows: torch.Tensor) -> bool:
     """Whether load_rows takes sources k / v for the cache rows k_rows / v_rows (all [B,T,KH,128]): not empty, one dtype and device,
-    16-byte aligned rows, no shared memory (the source may be a view of a cache), nothing traced."""
-    ts = (k, v, k_rows, v_rows)
-    if not untraced(*ts) or any(t.shape != k_rows.shape or t.dtype != k_rows.dtype or not t.is_cuda or t.device != k_rows.device for t in ts):
+    16-byte aligned rows, sources apart from the rows in memory (a source may be a view of a cache), nothing traced."""
+    shape, dtype = k_rows.shape, k_rows.dtype
+    es = _ROW_BYTES.get(dtype)
+    if es is None or len(shape) != 4 or shape[3] != 128 or not untraced(k, v, k_rows, v_rows):
         return False
-    if k_rows.dim() != 4 or k_rows.shape[3] != 128 or k_rows.numel() == 0 or k_rows.shape[0] > 65535 or k_rows.dtype not in (torch.bfloat16, torch.float16, torch.float32):
+    B, T, KH, _ = shape
+    if not (0 < B <= 65535 and T > 0 and KH > 0):
         return False
-    if any(st % (16 // t.element_size()) for t in ts for st in t.stride()[:3]) or any(t.stride(3) != 1 or t.data_ptr() % 16 for t in ts):
+    device, at = k_rows.device, []
+    for t in (k, v, k_rows, v_rows):
+        sb, st, sh, sd = t.stride() if t.dim() == 4 else (0, 0, 0, 0)
+        p = t.data_ptr() if t.is_cuda else 1
+        if p % 16 or sd != 1 or (sb | st | sh) * es % 16 or t.shape != shape or t.dtype != dtype or t.device != device or t.is_conj() or t.is_neg():
+            return False
+        at.append((p, p + ((B - 1) * sb + (T - 1) * st + (KH - 1) * sh + 128) * es))
+    sb, st, sh, _ = k_rows.stride()
+    if k_rows.stride() != v_rows.stride() or (KH > 1 and sh < 128) or (T > 1 and st < 128) or (B > 1 and sb < 128):
         return False
-    if any(t.is_conj() or t.is_neg() for t in ts):
-        return False
-    dst = {t.untyped_storage().data_ptr() for t in (k_rows, v_rows)}
-    B, T, KH, _ = k_rows.shape
-    distinct = all((KH == 1 or t.stride(2) >= 128) and (T == 1 or t.stride(1) >= 128) and (B == 1 or t.stride(0) >= 128) for t in (k_rows, v_rows))
-    return distinct and k_rows.stride() == v_rows.stride() and k.untyped_storage().data_ptr() not in dst and v.untyped_storage().data_ptr() not in dst
+    return all(hi <= lo2 or hi2 <= lo for lo, hi in at[:2] for lo2, hi2 in at[2:])
 
 
 def load_rows(k: torch.Tensor, v: torch.Tensor, k_rows: torch.Tensor, v_rows: torch.Tensor, params: Optional[HashParams] = None,

@@ -22,6 +22,12 @@ from ._lib import GQA_BLOCKED
 from .workloads import budget
 
 
+# Rows without codes: below this many bytes of keys two torch copies are done sooner, as their host work is less (13 us a call against
+# 22): 8 MB of keys 20 us (fp32: 16) against 22, 12.6 MB 25 (fp32: 21) against 22, 17 MB 29 (fp32: 25) against 22. With
+# codes one call to the library is the shorter way at every size (27 us against 28 and more from 1024 rows up).
+LOAD_ROWS_MIN_BYTES = 13 << 20
+
+
 @dataclass
 class SessionConfig:
     batch: int
@@ -91,11 +97,11 @@ class DecodeSession:
         their codes with the layer's key hash."""
         T = k.shape[1]
         k_rows, v_rows = self.k_cache[layer][:, start:start + T], self.v_cache[layer][:, start:start + T]
-        if ops.load_rows_covers(k, v, k_rows, v_rows):
+        if (codes or k.numel() * k.element_size() >= LOAD_ROWS_MIN_BYTES) and ops.load_rows_covers(k, v, k_rows, v_rows):
             ops.load_rows(k, v, k_rows, v_rows, self.hash_k[layer] if codes else None,
                           self.codes[layer][:, start:start + T] if codes else None)
             return
-        # host tensors, other dtypes, broadcast or overlapping sources: torch's copy
+        # few rows without codes, host tensors, other dtypes, broadcast or overlapping sources: torch's copy
         k_rows[:] = k
         v_rows[:] = v
         if codes:

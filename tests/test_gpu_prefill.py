@@ -201,6 +201,32 @@ def test_load_context_of_nothing_and_of_very_many_batch_rows(B, T):
     assert torch.equal(s.k_cache[0][:, :T], k) and torch.equal(s.v_cache[0][:, :T], v)
 
 
+@pytest.mark.parametrize("T,codes,one_call", [(50, False, False), (6655, False, False), (6656, False, True), (50, True, True)])
+def test_load_context_leaves_few_rows_without_codes_to_torchs_copies(T, codes, one_call, monkeypatch):
+    from spotlight_b200 import ops
+    from spotlight_b200.session import DecodeSession, SessionConfig
+    gen = torch.Generator(device="cuda").manual_seed(14)
+    h = [_hash("linear", 8, gen)]
+    s = DecodeSession(SessionConfig(1, 8, 8, 1, T + 7), h, h)
+    calls, load_rows = [], ops.load_rows
+    monkeypatch.setattr(ops, "load_rows", lambda *a: (calls.append(1), load_rows(*a)))
+    k, v = (torch.randn((1, T, 8, 128), generator=gen, device="cuda").bfloat16() for _ in range(2))
+    s.load_context(0, k, v, 3, codes=codes)
+    assert bool(calls) == one_call
+    assert torch.equal(s.k_cache[0][:, 3:3 + T], k) and torch.equal(s.v_cache[0][:, 3:3 + T], v)
+
+
+@pytest.mark.parametrize("apart", [True, False])
+def test_load_rows_covers_a_source_apart_from_the_rows(apart):
+    from spotlight_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(15)
+    kc, vc = _caches(2, 100, 4, True, gen)
+    src = slice(0, 40) if apart else slice(21, 61)
+    one = [x[:1] for x in (kc, vc)]                            # of several batch rows the address ranges cross
+    assert ops.load_rows_covers(one[0][:, src], one[1][:, src], one[0][:, 60:100], one[1][:, 60:100]) == apart
+    assert not ops.load_rows_covers(kc[:, src], vc[:, src], kc[:, 60:100], vc[:, 60:100])
+
+
 def test_load_context_fills_codes_held_as_signed_words():
     from spotlight_b200.session import DecodeSession, SessionConfig
     gen = torch.Generator(device="cuda").manual_seed(13)
