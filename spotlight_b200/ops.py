@@ -559,8 +559,9 @@ def decode_layer(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, hash_q: Hash
     B, QH, D = q.shape
     KH, n = k.shape[1], pos + 1
     assert D == 128
-    dev = _cuda(q, code_cache)
+    dev = _cuda(q, code_cache, k_cache, v_cache)
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+    assert k_cache.shape[2] == KH and v_cache.shape[2] == KH
     assert code_cache.shape[0] == B and code_cache.shape[2:] == (KH, 4)
     assert pos < code_cache.shape[1], "code cache is full"
     assert pos < k_cache.shape[1], "kv cache is full"

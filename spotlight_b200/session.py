@@ -177,21 +177,30 @@ class DecodeSession:
             return False
         if not (len(self.codes) == len(self.k_cache) == len(self.v_cache) == len(self.hash_q) == len(self.hash_k) == L):
             return False
+        dev, rows, words = self.q_in.device, (c.batch, c.kv_heads, 128), (c.batch, c.kv_heads, 4)
         ks, cs, kn, cn = self.k_cache[0].stride(), self.codes[0].stride(), self.k_cache[0].shape, self.codes[0].shape
-        if kn[1] <= pos or cn[1] <= pos or cn[2:] != (c.kv_heads, 4) or cs[1:] != (c.kv_heads * 4, 4, 1) or ks[3] != 1:
+        if not self.q_in.is_cuda or len(kn) != 4 or len(cn) != 4 or kn[1] <= pos or cn[1] <= pos or (kn[0], *kn[2:]) != rows or (cn[0], *cn[2:]) != words:
+            return False
+        if cs[1:] != (c.kv_heads * 4, 4, 1) or (c.batch == 1 and cs[0] < cn[1] * c.kv_heads * 4) or ks[3] != 1:
             return False
         for k, v, codes in zip(self.k_cache, self.v_cache, self.codes):
             if k.stride() != ks or v.stride() != ks or codes.stride() != cs or k.shape != kn or v.shape != kn or codes.shape != cn \
-                    or k.dtype != dt or v.dtype != dt or not k.is_cuda:
+                    or k.dtype != dt or v.dtype != dt or k.device != dev or v.device != dev or codes.device != dev:
                 return False
         for t, h in ((self.q_in, c.q_heads), (self.k_in, c.kv_heads), (self.v_in, c.kv_heads), (self.out, c.q_heads)):
-            if t.shape != (L, c.batch, h, 128) or t.dtype != dt or not t.is_contiguous() or not t.is_cuda:
+            if t.shape != (L, c.batch, h, 128) or t.dtype != dt or not t.is_contiguous() or t.device != dev:
                 return False
+        lists = [self.idx]
         if self.lru is not None and self.use_lru:
             rs = self.lru[0].k.stride()
-            if len(self.lru) != L or any((t.C, t.n_max, t.k.stride(), t.v.stride()) != (c.lru_slots, c.capacity, rs, rs) for t in self.lru):
+            if len(self.lru) != L or any((t.B, t.KH, t.C, t.n_max, t.k.dtype, t.k.stride(), t.v.stride()) !=
+                                         (c.batch, c.kv_heads, c.lru_slots, c.capacity, dt, rs, rs) for t in self.lru):
                 return False
-        return self.idx.is_contiguous() and self.idx.shape[:2] == (c.batch, c.kv_heads)
+            lists.append(self.slots)
+        for t in (*lists, self.cnt):
+            if t.dtype != torch.int32 or not t.is_contiguous() or t.device != dev or t.shape[:2] != (c.batch, c.kv_heads):
+                return False
+        return all(t.shape == self.idx.shape for t in lists) and self.cnt.dim() == 2
 
     def _step_in_one_call(self, pos: int):
         import ctypes as C

@@ -63,6 +63,38 @@ def test_step_takes_the_layer_steps_where_one_call_does_not_serve():
     assert not s._one_call(300)
 
 
+# buffers a caller exchanged: what the calls of layer_step refuse (or serve with another geometry) is left to them
+@pytest.mark.parametrize("what", ["codes", "heads", "batch", "idx", "cnt", "list", "slots", "table", "shape"])
+def test_one_call_leaves_exchanged_buffers_to_the_layer_steps(what):
+    from spotlight_b200 import ops
+    n = 300
+    s, _ = _session(10, 2, 4, 4, 1, n, torch.bfloat16, lru_slots=200)
+    s.set_position(n, 10000.0)
+    assert s._one_call(n)
+    if what == "codes":
+        s.codes = [s.codes[0][:1].clone()]                         # one batch row for two
+    elif what == "heads":
+        s.k_cache, s.v_cache = ([x[0][:, :, :2].contiguous()] for x in (s.k_cache, s.v_cache))
+    elif what == "batch":
+        s.k_cache, s.v_cache = ([x[0][:1].contiguous()] for x in (s.k_cache, s.v_cache))
+    elif what == "idx":
+        s.idx = s.idx.long()
+    elif what == "cnt":
+        s.cnt = s.cnt.long()
+    elif what == "list":
+        s.idx = s.idx[:, :, :0]
+    elif what == "slots":
+        s.slots = s.slots[:, :, :5].contiguous()
+    elif what == "table":
+        s.lru = [ops.LruTable(1, 4, n + 8, 200, torch.bfloat16, "cuda", fused=True)]
+    elif what == "shape":
+        s.codes = [s.codes[0].flatten(2)]
+    assert not s._one_call(n)
+    if what in ("codes", "idx"):
+        with pytest.raises(AssertionError):
+            s.step(n)
+
+
 # what Python's budget rule takes: integers beyond 32 bits ("never prune"), a budget above and below the other term, numbers that
 # are no int, a mask_out that leaves more than every key
 @pytest.mark.parametrize("mask_out,min_remain", [(0.9, sys.maxsize), (0.9, 2 ** 31), (0.9, 2 ** 32 + 5), (0.9, 20.5), (np.float32(0.9), 20), (1, 33), (0, 20),
