@@ -29,6 +29,8 @@
 // Every wait on an mbarrier is bounded; a wait that runs out raises the library's hash status word, the CTA lets its
 // copies in flight land, frees its TMEM and returns.
 // Same arithmetic as the warp-level kernel in sl_hash_mma.cu up to the order of the fp32 additions.
+#include <mutex>
+
 #include "sl_common.cuh"
 #include "sl_tc.cuh"
 
@@ -514,13 +516,22 @@ namespace sl {
 
 void set_hash_kernel(int mode) { g_hash_kernel = mode; }
 
-// The status word as the current device addresses it (null: none to be had).
+// The status word as the current device addresses it (null: none to be had). The first call may come from any thread and inside a
+// stream capture, which forbids an allocation unless the thread says that it is none of the capture's business.
 int* tc_status_word() {
-    if (!g_status_host) {
-        int* p = nullptr;
-        if (cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        *p = 0;
-        g_status_host = p;
+    static std::mutex mu;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!g_status_host) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            int* p = nullptr;
+            const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
+            *p = 0;
+            g_status_host = p;
+        }
     }
     int* d_status = nullptr;
     if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&d_status), g_status_host, 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }

@@ -1,4 +1,6 @@
 """RoPE + append and the causal attention of a prompt (tcgen05) against plain PyTorch, and against the general path."""
+import subprocess
+import sys
 import types
 
 import pytest
@@ -214,6 +216,31 @@ def test_load_context_leaves_few_rows_without_codes_to_torchs_copies(T, codes, o
     s.load_context(0, k, v, 3, codes=codes)
     assert bool(calls) == one_call
     assert torch.equal(s.k_cache[0][:, 3:3 + T], k) and torch.equal(s.v_cache[0][:, 3:3 + T], v)
+
+
+@pytest.mark.parametrize("call", ["hash", "attention", "load"])
+def test_the_first_call_of_a_process_may_be_inside_a_capture(call):
+    """In a process of its own: the library's first tensor-core call allocates its status word."""
+    code = f"""
+import torch
+from spotlight_b200 import ops
+torch.manual_seed(0)
+r = lambda *s: torch.randn(s, device="cuda").bfloat16()
+h, x, q, kv, codes = ops.HashParams([r(4, 128, 128)]), r(1, 300, 4, 128), r(1, 300, 8, 128), r(1, 300, 4, 2, 128), torch.zeros((1, 300, 4, 4), dtype=torch.int32, device="cuda")
+rows = kv[:, :, :, 0], kv[:, :, :, 1]
+run = dict(hash=lambda: ops.hash_encode(x, h).view(torch.int32), attention=lambda: ops.prefill_attention(q, *rows, 0),
+           load=lambda: (ops.load_rows(x, x, *rows, h, codes), codes)[1])["{call}"]
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    out = run()
+g.replay()
+got = out.clone()
+assert torch.equal(got, run())
+ops.check_status()
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 @pytest.mark.parametrize("apart", [True, False])
