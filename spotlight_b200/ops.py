@@ -80,26 +80,80 @@ def _kv_layout(t: torch.Tensor, list_heads_per_kv_head: int = 1) -> "_lib.KvLayo
 
 # ----------------------------------------------------------------------------- workspaces
 class _Workspaces:
-    """Zero-initialised scratch buffers, one per (kind, device, shape); the kernels leave
-    them zeroed, so they are allocated once and reused. A status word rides along."""
+    """Zero-initialised scratch buffers, one per (kind, device, shape, stream); the kernels leave
+    them zeroed, so they are allocated once and reused. A status word rides along.
+
+    The kernels keep counters, histograms and partial results in them, so that calls on two streams must not share one. At most
+    MAX_STREAMS buffers of a kind and shape are kept, the oldest goes first: its memory returns to its stream, in stream order.
+    A capture takes its stream's buffer, or else the one of that kind and shape that was used last, which is its warm-up's. What a
+    capture (or a caller that says `keep`) took stays until reset()."""
+
+    MAX_STREAMS = 8
 
     def __init__(self):
-        self._bufs = {}
+        self._bufs = {}              # (kind, device, shape) -> {stream: buffer and status word}, in the order they were made
+        self._last = {}              # (kind, device, shape) -> stream of the last call
+        self._kept = set()           # (kind, device, shape, stream) of the buffers that a graph replays with
+        self._outgrown = []          # (key, buffer and status word) of those that a larger one has replaced
 
-    def get(self, kind: str, device: torch.device, nbytes: int, shape=()) -> Tuple[torch.Tensor, torch.Tensor]:
+    def get(self, kind: str, device: torch.device, nbytes: int, shape=(), keep: bool = False) -> Tuple[torch.Tensor, torch.Tensor]:
         """`shape` = (B, KH, QH): the library lays a workspace out per shape and only guarantees
         to leave it zeroed for that shape, so every shape gets its own buffer."""
-        key = (kind, device, tuple(shape))
-        cur = self._bufs.get(key)
+        if device.index is None:
+            device = _indexed(device)
+        stream = torch._C._cuda_getCurrentRawStream(device.index)
+        what = (kind, device, shape)
+        bufs = self._bufs.setdefault(what, {})
+        cur = bufs.get(stream)
+        capturing = torch._C._cuda_isCurrentStreamCapturing()
+        if capturing and cur is None and bufs:
+            stream = self._last[what]
+            cur = bufs.get(stream)
         if cur is None or cur[0].numel() < nbytes:
-            buf = torch.zeros(max(nbytes, 256), dtype=torch.uint8, device=device)
-            status = torch.zeros(1, dtype=torch.int32, device=device)
-            cur = (buf, status)
-            self._bufs[key] = cur
+            if capturing:
+                stream = torch._C._cuda_getCurrentRawStream(device.index)
+            cur = self._new(what, stream, nbytes)
+        if capturing or keep:
+            self._kept.add((*what, stream))
+        self._last[what] = stream
         return cur
 
+    def _new(self, what, stream, nbytes):
+        bufs = self._bufs[what]
+        if (*what, stream) in self._kept and stream in bufs:
+            self._outgrown.append(((*what, stream), bufs[stream]))
+        cur = (torch.zeros(max(nbytes, 256), dtype=torch.uint8, device=what[1]), torch.zeros(1, dtype=torch.int32, device=what[1]))
+        bufs.pop(stream, None)
+        bufs[stream] = cur
+        free = [s for s in bufs if (*what, s) not in self._kept]
+        for s in free[: max(0, len(free) - self.MAX_STREAMS)]:
+            del bufs[s]
+        return cur
+
+    def _all(self):
+        return [((*what, s), cur) for what, bufs in self._bufs.items() for s, cur in bufs.items()] + self._outgrown
+
+    def status_words(self, device=None):
+        """(key, status word) of every buffer in use."""
+        return [(key, cur[1]) for key, cur in self._all() if device is None or key[1] == _indexed(torch.device(device))]
+
+    def clean(self, key):
+        """After a wait that ran out the counters are no longer to be trusted: the next call starts from a clean buffer."""
+        if key not in self._kept:
+            self._bufs[key[:3]].pop(key[3], None)
+            return
+        for k, cur in self._all():                                 # a graph's: cleaned where it is
+            if k == key:
+                cur[0].zero_()
+                cur[1].zero_()
+        torch.cuda.synchronize(key[1])
+
     def reset(self):
-        self._bufs.clear()
+        self.__init__()
+
+
+def _indexed(device: torch.device) -> torch.device:
+    return torch.device("cuda", torch.cuda.current_device()) if device.type == "cuda" and device.index is None else device
 
 
 workspaces = _Workspaces()
@@ -115,12 +169,10 @@ def check_status(device=None) -> None:
     """Host-side read of every status word (synchronises). Raises if a bounded device-side wait
     ran out; the affected workspace is dropped so the next call starts from a clean one."""
     bad = []
-    for key, (buf, status) in list(workspaces._bufs.items()):
-        if device is not None and key[1] != torch.device(device):
-            continue
+    for key, status in workspaces.status_words(device):
         if int(status.item()) != 0:
             bad.append((key, int(status.item())))
-            del workspaces._bufs[key]
+            workspaces.clean(key)
     hs = int(_lib.lib.sl_hash_status())
     if hs != 0:
         bad.append((("hash_encode",), hs))

@@ -12,12 +12,13 @@ This is the host-side counterpart of the reference's per-layer loop
 (spotlight/modifiers/gpu_cache.py) for callers that drive the attention path themselves."""
 from __future__ import annotations
 
+import ctypes as C
 from dataclasses import dataclass
 from typing import List, Optional
 
 import torch
 
-from . import ops
+from . import _lib, ops
 from ._lib import GQA_BLOCKED
 from .workloads import budget
 
@@ -85,6 +86,7 @@ class DecodeSession:
             self.slots = torch.empty_like(self.idx)
         self.use_lru = self.lru is not None      # stage 3 can be switched off to time the three-stage step on the same caches
         self._graphs = {}
+        self._side = None                        # stream of the warm-ups before captures
         self._host = None
         # device-side position: one captured step serves every token (see step_dev)
         self.pos_dev = torch.zeros((1,), dtype=torch.int64, device=dev)
@@ -171,47 +173,43 @@ class DecodeSession:
         c = self.cfg
         if c.fix_layers or not 0 <= pos < c.capacity or type(self).layer_step is not DecodeSession.layer_step or "layer_step" in self.__dict__:
             return False
-        L, dt = c.layers, self.q_in.dtype
+        B, QH, KH, L = c.batch, c.q_heads, c.kv_heads, c.layers
         k_budget = budget(pos + 1, c.mask_out, c.min_remain)
         if type(k_budget) is not int or k_budget < 0:
             return False
         if not (len(self.codes) == len(self.k_cache) == len(self.v_cache) == len(self.hash_q) == len(self.hash_k) == L):
             return False
-        dev, rows, words = self.q_in.device, (c.batch, c.kv_heads, 128), (c.batch, c.kv_heads, 4)
+        dt, dev = self.q_in.dtype, self.q_in.get_device()              # get_device(): -1 for a host tensor
         ks, cs, kn, cn = self.k_cache[0].stride(), self.codes[0].stride(), self.k_cache[0].shape, self.codes[0].shape
-        if not self.q_in.is_cuda or len(kn) != 4 or len(cn) != 4 or kn[1] <= pos or cn[1] <= pos or (kn[0], *kn[2:]) != rows or (cn[0], *cn[2:]) != words:
+        if dev < 0 or len(kn) != 4 or len(cn) != 4 or kn[1] <= pos or cn[1] <= pos or kn != (B, kn[1], KH, 128) or cn != (B, cn[1], KH, 4):
             return False
-        if cs[1:] != (c.kv_heads * 4, 4, 1) or (c.batch == 1 and cs[0] < cn[1] * c.kv_heads * 4) or ks[3] != 1:
+        if cs[1:] != (KH * 4, 4, 1) or (B == 1 and cs[0] < cn[1] * KH * 4) or ks[3] != 1:
             return False
         for k, v, codes in zip(self.k_cache, self.v_cache, self.codes):
             if k.stride() != ks or v.stride() != ks or codes.stride() != cs or k.shape != kn or v.shape != kn or codes.shape != cn \
-                    or k.dtype != dt or v.dtype != dt or k.device != dev or v.device != dev or codes.device != dev:
+                    or k.dtype != dt or v.dtype != dt or not k.get_device() == v.get_device() == codes.get_device() == dev:
                 return False
-        for t, h in ((self.q_in, c.q_heads), (self.k_in, c.kv_heads), (self.v_in, c.kv_heads), (self.out, c.q_heads)):
-            if t.shape != (L, c.batch, h, 128) or t.dtype != dt or not t.is_contiguous() or t.device != dev:
+        for t, h in ((self.q_in, QH), (self.k_in, KH), (self.v_in, KH), (self.out, QH)):
+            if t.shape != (L, B, h, 128) or t.dtype != dt or not t.is_contiguous() or t.get_device() != dev:
                 return False
-        lists = [self.idx]
+        cap = self.idx.shape[-1]
+        lists = [(self.idx, (B, KH, cap)), (self.cnt, (B, KH))]
         if self.lru is not None and self.use_lru:
             rs = self.lru[0].k.stride()
             if len(self.lru) != L or any((t.B, t.KH, t.C, t.n_max, t.k.dtype, t.k.stride(), t.v.stride()) !=
-                                         (c.batch, c.kv_heads, c.lru_slots, c.capacity, dt, rs, rs) for t in self.lru):
+                                         (B, KH, c.lru_slots, c.capacity, dt, rs, rs) for t in self.lru):
                 return False
-            lists.append(self.slots)
-        for t in (*lists, self.cnt):
-            if t.dtype != torch.int32 or not t.is_contiguous() or t.device != dev or t.shape[:2] != (c.batch, c.kv_heads):
-                return False
-        return all(t.shape == self.idx.shape for t in lists) and self.cnt.dim() == 2
+            lists.append((self.slots, (B, KH, cap)))
+        return all(t.shape == shape and t.dtype == torch.int32 and t.is_contiguous() and t.get_device() == dev for t, shape in lists)
 
     def _step_in_one_call(self, pos: int):
-        import ctypes as C
-        from . import _lib
         c, L, n = self.cfg, self.cfg.layers, pos + 1
         ops._cuda(self.q_in)
         a, keep = self._step_args()                  # from the buffers as they are now
         ops.step_budget(a, budget(n, c.mask_out, c.min_remain), n)
         shape = (c.batch, c.kv_heads, c.q_heads)
-        sw, status = ops.workspaces.get("scan", self.device, _lib.lib.sl_scan_topk_workspace_bytes(c.batch, n, c.kv_heads, c.q_heads), shape)
-        aw, _ = ops.workspaces.get("attn", self.device, _lib.lib.sl_sparse_attn_workspace_bytes(c.batch, c.kv_heads, c.q_heads), shape)
+        sw, status = self._scan_workspace()
+        aw, _ = ops.workspaces.get("attn", self.q_in.device, _lib.lib.sl_sparse_attn_workspace_bytes(c.batch, c.kv_heads, c.q_heads), shape)
         a.d_scan_workspace, a.scan_workspace_bytes, a.d_status = sw.data_ptr(), sw.numel(), status.data_ptr()
         a.d_attn_workspace, a.attn_workspace_bytes = aw.data_ptr(), aw.numel()
         clocks = stats = None
@@ -233,8 +231,6 @@ class DecodeSession:
     def _step_args(self):
         """The argument block of sl_decode_step over this session's buffers, without the budget and the workspaces, and what it
         points to."""
-        import ctypes as C
-        from . import _lib
         c, L = self.cfg, self.cfg.layers
         arr = lambda ts: (C.c_void_p * L)(*[t.data_ptr() for t in ts])
 
@@ -273,7 +269,6 @@ class DecodeSession:
         return a, keep
 
     def _native_args(self):
-        from . import _lib
         c = self.cfg
         assert not c.fix_layers
         if getattr(self, "_native", None) is None:
@@ -282,10 +277,9 @@ class DecodeSession:
             a, keep = self._step_args()
             a.min_remain, a.mask_out = min(c.min_remain, c.capacity), c.mask_out     # no context is longer; a larger integer would wrap
             shape = (c.batch, c.kv_heads, c.q_heads)
-            sw, status = ops.workspaces.get("scan", self.device, _lib.lib.sl_scan_topk_workspace_bytes(
-                c.batch, c.capacity, c.kv_heads, c.q_heads), shape)
-            aw, _ = ops.workspaces.get("attn", self.device, _lib.lib.sl_sparse_attn_workspace_bytes(
-                c.batch, c.kv_heads, c.q_heads), shape)
+            sw, status = self._scan_workspace(keep=True)           # the block is kept, and with it what it points to
+            aw, _ = ops.workspaces.get("attn", self.q_in.device, _lib.lib.sl_sparse_attn_workspace_bytes(
+                c.batch, c.kv_heads, c.q_heads), shape, keep=True)
             a.d_scan_workspace, a.scan_workspace_bytes = sw.data_ptr(), sw.numel()
             a.d_attn_workspace, a.attn_workspace_bytes = aw.data_ptr(), aw.numel()
             a.d_status = status.data_ptr()
@@ -299,8 +293,6 @@ class DecodeSession:
     def step_native(self, pos: int):
         """`step(pos)` with the layer loop in the library (sl_decode_step): one call per token instead
         of three per layer."""
-        import ctypes as C
-        from . import _lib
         _lib.check(_lib.lib.sl_decode_step(C.byref(self._native_args()), pos,
                                            torch.cuda.current_stream(self.device).cuda_stream))
         ops.launch_count += (6 if self.use_lru else 4) * self.cfg.layers
@@ -309,8 +301,6 @@ class DecodeSession:
         """One token at the position held in `self.pos_dev` (device memory): the launches depend on no
         host-side position, so a captured graph of this call serves every token of a decode loop
         (capture_dev). Needs set_position_table to cover the positions that will be visited."""
-        import ctypes as C
-        from . import _lib
         assert self.cos_tab is not None, "call set_position_table first"
         d = _lib.DecodeDev()
         d.d_pos = self.pos_dev.data_ptr()
@@ -340,15 +330,10 @@ class DecodeSession:
             self.step_dev(max_context)
             if host_io:
                 self._host["out"].copy_(self.out, non_blocking=True)
-                self._host["status"].copy_(self._scan_status(), non_blocking=True)
+                self._host["status"].copy_(self._native[self.use_lru][4], non_blocking=True)
 
         saved = self.pos_dev.clone()
-        s = torch.cuda.Stream(device=self.device)
-        s.wait_stream(torch.cuda.current_stream(self.device))
-        with torch.cuda.stream(s):
-            run()
-        torch.cuda.current_stream(self.device).wait_stream(s)
-        torch.cuda.synchronize(self.device)
+        self._warm_up(run)
         self.pos_dev.copy_(saved)
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
@@ -365,12 +350,7 @@ class DecodeSession:
             return self._graphs[key]
         if host_io:
             self._ensure_host()
-        s = torch.cuda.Stream(device=self.device)
-        s.wait_stream(torch.cuda.current_stream(self.device))
-        with torch.cuda.stream(s):
-            self._run(pos, stage, host_io)            # warm-up outside capture (workspaces allocate here)
-        torch.cuda.current_stream(self.device).wait_stream(s)
-        torch.cuda.synchronize(self.device)
+        self._warm_up(lambda: self._run(pos, stage, host_io))
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             self._run(pos, stage, host_io)
@@ -385,14 +365,24 @@ class DecodeSession:
         self.step(pos, stage)
         if host_io:
             self._host["out"].copy_(self.out, non_blocking=True)
-            self._host["status"].copy_(self._scan_status(), non_blocking=True)   # rides along with the outputs
+            self._host["status"].copy_(self._scan_workspace()[1], non_blocking=True)   # rides along with the outputs
 
-    def _scan_status(self) -> torch.Tensor:
-        """The status word of the scan workspace this session's steps use (set by a bounded wait that ran out)."""
-        from . import _lib
+    def _scan_workspace(self, keep: bool = False):
+        """The scan workspace of this session's steps on the current stream, sized for its capacity, and its status word (set by a
+        bounded wait that ran out)."""
         c = self.cfg
         need = _lib.lib.sl_scan_topk_workspace_bytes(c.batch, c.capacity, c.kv_heads, c.q_heads)
-        return ops.workspaces.get("scan", self.device, need, (c.batch, c.kv_heads, c.q_heads))[1]
+        return ops.workspaces.get("scan", self.q_in.device, need, (c.batch, c.kv_heads, c.q_heads), keep)
+
+    def _warm_up(self, run):
+        """`run` once outside a capture, on a stream of the session's own: workspaces are allocated there and the capture takes them."""
+        if self._side is None:
+            self._side = torch.cuda.Stream(device=self.device)
+        self._side.wait_stream(torch.cuda.current_stream(self.device))
+        with torch.cuda.stream(self._side):
+            run()
+        torch.cuda.current_stream(self.device).wait_stream(self._side)
+        torch.cuda.synchronize(self.device)
 
     # ------------------------------------------------------------------ host buffers
     def _ensure_host(self):
