@@ -669,7 +669,6 @@ WsLayout ws_layout(int B, long long N, int KH, int G, bool with_hist, bool spill
     w.hist_off = off; if (with_hist) off = align_up(off + (size_t)NCOPY * B * KH * (nbins > 0 ? nbins : 128 * G + 1) * 4, 256);
     w.chist_off = off; if (with_hist) off = align_up(off + (size_t)NCOPY * B * KH * 32 * 4, 256);
     w.seg_off = off; off = align_up(off + (size_t)B * max_cpb * KH * 16, 256);
-    w.score_off = off; if (spill) off = align_up(off + (size_t)B * N * KH * 2, 256);
     w.epoch_off = w.chist2_off = w.pub_off = w.puba_off = w.wsc_off = off;
     if (with_hist && (nbins <= 0 || slscan::lean_nc(nbins) <= 32 * slscan::LEAN_CPL_MAX)) {
         const int nb = nbins > 0 ? nbins : 128 * G + 1;
@@ -679,6 +678,8 @@ WsLayout ws_layout(int B, long long N, int KH, int G, bool with_hist, bool spill
         w.puba_off = off; off = align_up(off + (size_t)std::max(B, sl::sm_count()) * KH * slscan::lean_nc(nb) * 2, 256);
         w.wsc_off = off; off = align_up(off + (size_t)B * KH * slscan::LEAN_MAX_WIN * 2, 256);
     }
+    // the only area whose size depends on N, and the only one a call need not leave zeroed: behind the others, whose places stay
+    w.score_off = off; if (spill) off = align_up(off + (size_t)B * N * KH * 2, 256);
     w.total = off;
     return w;
 }

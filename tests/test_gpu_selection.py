@@ -84,6 +84,26 @@ def test_topk_from_scores_clamps_to_the_given_range():
         assert torch.equal(a, b)
 
 
+def test_a_context_whose_scores_spill_leaves_the_workspace_to_a_shorter_one():
+    """The workspace of a shape serves every length: scores that do not fit on chip must not land where a shorter context's launch
+    keeps its counts."""
+    from spotlight_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(21)
+    B, KH, N, short = 37, 32, 13500, 3000                        # four CTAs per batch row, 3375 keys of 32 heads each: 216 KB of scores
+    words = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, generator=gen, device="cuda").to(torch.int32).view(torch.uint32)
+    q, codes = words(B, KH, 4), words(B, N, KH, 4)
+    ops.workspaces.reset()
+    want = [x.clone() for x in ops.scan_topk(q, codes[:, :short], 300)]
+    ops.workspaces.reset()
+    for _ in range(2):
+        ops.scan_topk(q, codes, 1350)
+        idx, cnt = ops.scan_topk(q, codes[:, :short], 300)
+        assert torch.equal(cnt, want[1])
+        valid = torch.arange(idx.shape[2], device="cuda") < cnt[..., None]
+        assert torch.equal(idx[valid], want[0][valid])
+    ops.check_status(torch.device("cuda", 0))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("B,N,KH,budget", [(1, 50, 3, 1), (2, 300, 4, 63), (3, 1000, 8, 129), (1, 65, 1, 65)])
 def test_gather_kv(B, N, KH, budget, dtype):
