@@ -341,9 +341,10 @@ int sl_lru_update(const int32_t* d_idx, int idx_capacity, const int32_t* d_cnt, 
 /* sl_lru_update with the cache geometries spelled out (backing store and resident buffers may be fused
  * K|V caches or host memory with any strides), an optional step in DEVICE memory (*d_step, e.g. the decode
  * position, so that a replayed CUDA graph advances the table's clock) and an optional workspace of
- * sl_lru_workspace_bytes(B, KH, idx_capacity) bytes, zero-filled once and left zeroed by every call: with it
+ * sl_lru_workspace_bytes(B, KH, idx_capacity) bytes, zero-filled once; every call leaves it ready for the next one with the same
+ * B and KH and any idx_capacity it is large enough for. With it
  * the update is spread over several CTAs per (b, kv head), each owning a slice of the index list and a range of the
- * slots (a cooperative launch; what the CTAs of a pair need from one another crosses the workspace behind four bounded
+ * slots (a cooperative launch; what the CTAs of a pair need from one another crosses the workspace behind three bounded
  * barriers of the pair; SL_OPT_LRU_MULTI_CTA = 0: only the probe is spread and the last CTA to finish handles the
  * misses alone). Results are those of sl_lru_update. */
 size_t sl_lru_workspace_bytes(int B, int KH, int idx_capacity);

@@ -717,15 +717,17 @@ int lru_launch(const int32_t* d_idx, int idx_capacity, const int32_t* d_cnt, int
                    "sl_lru_update_ex: workspace %zu < required %zu", workspace_bytes, sl_lru_workspace_bytes(B, KH, idx_capacity));
         SL_REQUIRE(sl::aligned16(d_workspace), SL_EALIGN, "sl_lru_update_ex: workspace not 16-byte aligned");
         a.parts = lru_parts(B, KH, idx_capacity);
-        a.g_count = static_cast<unsigned*>(d_workspace);
-        a.g_m = reinterpret_cast<int*>(a.g_count + (((size_t)B * KH * 2 + 63) / 64) * 64);
-        a.g_miss = reinterpret_cast<unsigned*>(a.g_m + (((size_t)B * KH + 63) / 64) * 64);
-        a.g_pairs = reinterpret_cast<int2*>(a.g_miss + (((size_t)B * KH * nw + 3) / 4) * 4);
-        // behind the pairs: what the CTAs of a pair exchange when all of them work through the update
+        // first what a call must find zeroed and leaves so, at places that do not depend on the list's capacity: a workspace serves
+        // lists of any length up to the one it was sized for
         const size_t bh = (size_t)B * KH;
+        a.g_count = static_cast<unsigned*>(d_workspace);
+        a.g_m = reinterpret_cast<int*>(a.g_count + ((bh * 2 + 63) / 64) * 64);
+        a.g_bar = reinterpret_cast<unsigned*>(a.g_m + ((bh + 63) / 64) * 64);
+        a.g_miss = a.g_bar + bh * 8;
+        a.g_pairs = reinterpret_cast<int2*>(a.g_miss + ((bh * nw + 3) / 4) * 4);
+        // behind the pairs: what the CTAs of a pair exchange when all of them work through the update
         a.g_hist = reinterpret_cast<unsigned*>(a.g_pairs + bh * idx_capacity);
-        a.g_bar = a.g_hist + ((bh * a.parts * NBIN + 3) / 4) * 4;
-        a.g_pm = reinterpret_cast<int*>(a.g_bar + bh * 8);
+        a.g_pm = reinterpret_cast<int*>(a.g_hist + ((bh * a.parts * NBIN + 3) / 4) * 4);
         a.g_vict = a.g_pm + bh * 64;
     }
     if (g_lru_multi && phase == 0 && d_workspace && a.parts > 1 && B * KH * a.parts <= sl::sm_count()) {
@@ -758,7 +760,7 @@ int lru_launch(const int32_t* d_idx, int idx_capacity, const int32_t* d_cnt, int
 extern "C" size_t sl_lru_workspace_bytes(int B, int KH, int idx_capacity) {
     if (B <= 0 || KH <= 0 || idx_capacity <= 0) return 0;
     const size_t nw = ((size_t)idx_capacity + 31) / 32;
-    // counters, misses per pair, miss bitmaps, {key, slot} pairs of the misses
+    // counters, misses per pair, (barrier counters, counted below), miss bitmaps, {key, slot} pairs of the misses
     const size_t bh = (size_t)B * KH;
     return ((((size_t)B * KH * 2 + 63) / 64) * 64 + (((size_t)B * KH + 63) / 64) * 64 + (((size_t)B * KH * nw + 3) / 4) * 4) * 4 +
            (size_t)B * KH * idx_capacity * 8 +

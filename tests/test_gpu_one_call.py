@@ -191,3 +191,26 @@ def test_an_overfull_lru_table_raises_its_status_and_the_attention_stays_in_boun
     s.step(n)
     if dtype == torch.bfloat16:
         assert torch.equal(s.out, out)
+
+
+@pytest.mark.parametrize("multi", [1, 0])
+def test_one_lru_workspace_serves_lists_of_any_capacity(multi):
+    """Long and short lists in turn (several CTAs per pair and one): the table whose workspace stays is the table that gets a new one."""
+    from spotlight_b200 import _lib, ops
+    gen = torch.Generator(device="cuda").manual_seed(30)
+    B, KH, n = 1, 4, 20000
+    k, v = (torch.randn((B, n, KH, 128), generator=gen, device="cuda").bfloat16() for _ in range(2))
+    a, b = (ops.LruTable(B, KH, n, 9000, torch.bfloat16, "cuda") for _ in range(2))
+    ops.configure(_lib.SL_OPT_LRU_MULTI_CTA, multi)
+    try:
+        for keep in (6000, 700, 6000, 3100, 2049, 8192, 40):
+            idx = torch.stack([torch.randperm(n, generator=gen, device="cuda")[:keep].sort().values for _ in range(KH)])[None].int()
+            cnt = torch.full((B, KH), keep, dtype=torch.int32, device="cuda")
+            b.ws = None
+            sa, sb = (ops.lru_update(t, idx, cnt, k, v) for t in (a, b))
+            assert torch.equal(sa, sb)
+            for x in ("k", "v", "tok2slot", "slot2tok", "last_used", "stats", "status"):
+                assert torch.equal(getattr(a, x), getattr(b, x)), (keep, x)
+            assert torch.equal(a.slot2tok.gather(2, sa.long()), idx)
+    finally:
+        ops.configure(_lib.SL_OPT_LRU_MULTI_CTA, 1)
