@@ -181,10 +181,13 @@ def test_an_overfull_lru_table_raises_its_status_and_the_attention_stays_in_boun
     for x in ("q_in", "k_in", "v_in"):
         getattr(s, x).copy_(torch.randn(getattr(s, x).shape, generator=gen, device="cuda"))
     s.set_position(n, 10000.0)
+    s.slots.fill_(2 ** 30)                                        # an entry the update does not write would show, and be read, as this
     s.step(n)
     torch.cuda.synchronize()
     assert [int(t.status) for t in s.lru] == [3, 3]
-    assert all(int(t.slot2tok.max()) == -1 and not t.k.any() for t in s.lru) or dtype == torch.float32
+    assert all(int(t.slot2tok.max()) == -1 and int(t.tok2slot.max()) == -1 and not t.k.any() and not t.v.any() for t in s.lru)
+    left = s.slots[torch.arange(s.slots.shape[2], device="cuda") < s.cnt[..., None]]
+    assert bool((left == (0 if dtype == torch.float32 else -2 ** 31)).all())       # any slot, or a miss without one
     ops.check_status(torch.device("cuda", 0))
     out = s.out.clone()
     s.use_lru = False
