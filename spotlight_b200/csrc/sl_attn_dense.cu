@@ -1,6 +1,6 @@
-// The tensor-core decode attention (sl_attn_mma.cuh) without an index list. A module of its own: with these forms beside the
-// others in one module (and the row copy beside the decode kernels of sl_hash.cu) the 32-layer decode step at 32K keys took
-// 807 us instead of 801 although the kernels it runs compile to the same registers: where their code lies on the device differs.
+// The tensor-core decode attention (sl_attn_mma.cuh) without an index list, a module of its own. The 32-layer decode step at 32K keys took
+// 807 us with these forms (and the row copy of sl_load.cu) in the decode kernels' modules and 801 - 805 with them apart, where
+// 801 - 805 had been measured before either: a difference of at most 1 %, whose cause is not known (the same registers).
 #include "sl_attn_mma.cuh"
 
 namespace sl {

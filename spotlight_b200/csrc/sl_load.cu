@@ -1,7 +1,7 @@
 // New rows into a layer's caches (sl_load_rows). Without their codes, or where the tensor-core kernel does not build them: K and V in one
 // launch, 16-byte pieces, four in flight per thread. Bound by its bytes: 131 072 x 8 rows of K and V (1.07 GB moved) in 177 us, 6.1 TB/s
 // (two strided torch copies: 594 us).
-// A module of its own: beside the decode kernels in sl_hash.cu it made the decode step slower (see sl_attn_dense.cu).
+// A module of its own (see sl_attn_dense.cu). Few rows without codes stay with two copies of the caller's (session.py).
 #include "sl_common.cuh"
 
 namespace {
