@@ -21,11 +21,11 @@
 //   EPI2  D2 -> registers, rounding points, sign bit of every value: a thread holds two 32-bit words of its
 //         row's code and stores them                            -> d2_free
 // Bound by the activation: two MUFU operations per hidden value, 4096 clocks per tile of 128 x 256, against 2048 of the tensor
-// core. 128 -> 256 -> 128, 131 072 x 8 rows: 171 us (267 with one tile in flight and a table of SiLU values in
-// shared memory); 128 -> 128 -> 128 residual: 150 us (231). The linear hash has a kernel of its own further
+// core. 128 -> 256 -> 128, 131 072 x 8 rows, contiguous or the K half of a fused cache: 171 us back to back (267 with one tile in
+// flight and a table of SiLU values in shared memory); 128 -> 128 -> 128 residual: 136 us (231). The linear hash has a kernel of its own further
 // down (one contraction per tile, bound by the stream of its input rows). With LOAD the input rows are new rows of a cache: the
 // K rows leave for it from the input stage, the V rows are copied beside them, all by TMA, and the cache is
-// not read back: 131 072 x 8 rows into a fused cache with their codes in 244 us, where two strided copies and the codes took 867.
+// not read back: 131 072 x 8 rows into a fused cache with their codes in 235 us, where two strided copies and the codes took 867.
 // Every wait on an mbarrier is bounded; a wait that runs out raises the library's hash status word, the CTA lets its
 // copies in flight land, frees its TMEM and returns.
 // Same arithmetic as the warp-level kernel in sl_hash_mma.cu up to the order of the fp32 additions.

@@ -17,8 +17,12 @@
 // (16 a clock and SM: 1024 clocks per 128 x 128 tile) and the tensor core (two contractions of 512) are each about half
 // busy; letting the two tiles' exponentials take turns changes nothing (136.4 us against 137).
 // Blocks are ordered longest first (the last rows of a prompt see the most keys), so the tail of the launch is short.
-// Measured (32 / 8 heads): 137 us for a prompt of 4001 tokens, 0.96 PFLOP/s of causal work, where torch's attention under the
-// same mask took 3 406 us.
+// Measured (32 / 8 heads): 131 us for a prompt of 4001 tokens, 1.00 PFLOP/s of causal work, where torch's attention under the
+// same mask took 3 406 us. The grid does not split the keys, so a short chunk over a long context fills few SMs (64 tokens: 8 CTAs); it
+// is still the shorter way (whole layer call, torch's path in brackets): 2 tokens over 32 000 keys 487 us (983), 64 over 32 000
+// 489 (991), 512 over 32 000 501 (1 010), 64 over 4 096 78 (189), 28 / 4 heads 64 over 120 000 1 780 (3 430).
+// Error against 64 bits: 1.00 of torch's over prompts of 64 to 4096 tokens with up to 700 keys before them, at most 1.04 where torch takes
+// its kernel with the exact maximum (1.20 with scores of deviation 4).
 // Every wait is bounded; one that runs out raises sl_hash_status, the CTA lets its copies land, frees its TMEM and returns.
 #include "sl_common.cuh"
 #include "sl_tc.cuh"

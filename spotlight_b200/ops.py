@@ -103,7 +103,9 @@ class _Workspaces:
             device = _indexed(device)
         stream = torch._C._cuda_getCurrentRawStream(device.index)
         what = (kind, device, shape)
-        bufs = self._bufs.setdefault(what, {})
+        bufs = self._bufs.get(what)
+        if bufs is None:
+            bufs = self._bufs[what] = {}
         cur = bufs.get(stream)
         capturing = torch._C._cuda_isCurrentStreamCapturing()
         if capturing and cur is None and bufs:
