@@ -5,6 +5,7 @@ All tensors must live on a CUDA device. There is no CPU path."""
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import List, Optional, Sequence, Tuple
 
 import torch
@@ -159,6 +160,13 @@ def _indexed(device: torch.device) -> torch.device:
 
 
 workspaces = _Workspaces()
+
+
+@functools.lru_cache(maxsize=256)
+def workspace_bytes(what: str, device: int, *shape: int) -> int:
+    """lib.sl_<what>_workspace_bytes(*shape) on the current device, whose index the caller names: a number of the shape and the device
+    alone (a call into the library takes longer than looking it up)."""
+    return getattr(lib, f"sl_{what}_workspace_bytes")(*shape)
 
 
 def configure(option: int, value: int) -> None:

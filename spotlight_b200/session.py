@@ -189,8 +189,9 @@ class DecodeSession:
             if k.stride() != ks or v.stride() != ks or codes.stride() != cs or k.shape != kn or v.shape != kn or codes.shape != cn \
                     or k.dtype != dt or v.dtype != dt or not k.get_device() == v.get_device() == codes.get_device() == dev:
                 return False
-        for t, h in ((self.q_in, QH), (self.k_in, KH), (self.v_in, KH), (self.out, QH)):
-            if t.shape != (L, B, h, 128) or t.dtype != dt or not t.is_contiguous() or t.get_device() != dev:
+        qs, kvs = (L, B, QH, 128), (L, B, KH, 128)
+        for t, shape in ((self.q_in, qs), (self.k_in, kvs), (self.v_in, kvs), (self.out, qs)):
+            if t.shape != shape or t.dtype != dt or not t.is_contiguous() or t.get_device() != dev:
                 return False
         cap = self.idx.shape[-1]
         lists = [(self.idx, (B, KH, cap)), (self.cnt, (B, KH))]
@@ -209,7 +210,8 @@ class DecodeSession:
         ops.step_budget(a, budget(n, c.mask_out, c.min_remain), n)
         shape = (c.batch, c.kv_heads, c.q_heads)
         sw, status = self._scan_workspace()
-        aw, _ = ops.workspaces.get("attn", self.q_in.device, _lib.lib.sl_sparse_attn_workspace_bytes(c.batch, c.kv_heads, c.q_heads), shape)
+        dev = self.q_in.device
+        aw, _ = ops.workspaces.get("attn", dev, ops.workspace_bytes("sparse_attn", dev.index, *shape), shape)
         a.d_scan_workspace, a.scan_workspace_bytes, a.d_status = sw.data_ptr(), sw.numel(), status.data_ptr()
         a.d_attn_workspace, a.attn_workspace_bytes = aw.data_ptr(), aw.numel()
         clocks = stats = None
@@ -232,11 +234,12 @@ class DecodeSession:
         """The argument block of sl_decode_step over this session's buffers, without the budget and the workspaces, and what it
         points to."""
         c, L = self.cfg, self.cfg.layers
-        arr = lambda ts: (C.c_void_p * L)(*[t.data_ptr() for t in ts])
+        P, H = C.c_void_p * L, _lib.HashParamsStruct * L
+        arr = lambda ts: P(*[t.data_ptr() for t in ts])
 
         def rows(t):                                 # the layers' slices of a [L, ...] tensor
             base, step = t.data_ptr(), t.stride(0) * t.element_size()
-            return (C.c_void_p * L)(*range(base, base + L * step, step))
+            return P(*range(base, base + L * step, step))
 
         a = _lib.DecodeStepArgs()
         a.B, a.QH, a.KH, a.layers = c.batch, c.q_heads, c.kv_heads, L
@@ -247,8 +250,7 @@ class DecodeSession:
         a.kv_batch_stride, a.kv_token_stride, a.kv_head_stride = kv.batch_stride, kv.token_stride, kv.head_stride
         keep = {"q": rows(self.q_in), "k": rows(self.k_in), "v": rows(self.v_in), "codes": arr(self.codes), "kc": arr(self.k_cache),
                 "vc": arr(self.v_cache), "out": rows(self.out),
-                "hq": (_lib.HashParamsStruct * L)(*[h.struct for h in self.hash_q]),
-                "hk": (_lib.HashParamsStruct * L)(*[h.struct for h in self.hash_k])}
+                "hq": H(*[h.struct for h in self.hash_q]), "hk": H(*[h.struct for h in self.hash_k])}
         a.d_q, a.d_k, a.d_v = keep["q"], keep["k"], keep["v"]
         a.hash_q, a.hash_k = keep["hq"], keep["hk"]
         a.d_code_cache, a.d_k_cache, a.d_v_cache, a.d_out = keep["codes"], keep["kc"], keep["vc"], keep["out"]
@@ -278,8 +280,8 @@ class DecodeSession:
             a.min_remain, a.mask_out = min(c.min_remain, c.capacity), c.mask_out     # no context is longer; a larger integer would wrap
             shape = (c.batch, c.kv_heads, c.q_heads)
             sw, status = self._scan_workspace(keep=True)           # the block is kept, and with it what it points to
-            aw, _ = ops.workspaces.get("attn", self.q_in.device, _lib.lib.sl_sparse_attn_workspace_bytes(
-                c.batch, c.kv_heads, c.q_heads), shape, keep=True)
+            dev = self.q_in.device
+            aw, _ = ops.workspaces.get("attn", dev, ops.workspace_bytes("sparse_attn", dev.index, *shape), shape, keep=True)
             a.d_scan_workspace, a.scan_workspace_bytes = sw.data_ptr(), sw.numel()
             a.d_attn_workspace, a.attn_workspace_bytes = aw.data_ptr(), aw.numel()
             a.d_status = status.data_ptr()
@@ -370,9 +372,9 @@ class DecodeSession:
     def _scan_workspace(self, keep: bool = False):
         """The scan workspace of this session's steps on the current stream, sized for its capacity, and its status word (set by a
         bounded wait that ran out)."""
-        c = self.cfg
-        need = _lib.lib.sl_scan_topk_workspace_bytes(c.batch, c.capacity, c.kv_heads, c.q_heads)
-        return ops.workspaces.get("scan", self.q_in.device, need, (c.batch, c.kv_heads, c.q_heads), keep)
+        c, dev = self.cfg, self.q_in.device
+        need = ops.workspace_bytes("scan_topk", dev.index, c.batch, c.capacity, c.kv_heads, c.q_heads)
+        return ops.workspaces.get("scan", dev, need, (c.batch, c.kv_heads, c.q_heads), keep)
 
     def _warm_up(self, run):
         """`run` once outside a capture, on a stream of the session's own: workspaces are allocated there and the capture takes them."""
