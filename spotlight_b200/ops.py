@@ -177,7 +177,7 @@ def configure(option: int, value: int) -> None:
 
 def check_status(device=None) -> None:
     """Host-side read of every status word (synchronises). Raises if a bounded device-side wait
-    ran out; the affected workspace is dropped so the next call starts from a clean one."""
+    ran out; the affected workspace is dropped (one that a graph replays with is zeroed) so the next call starts from a clean one."""
     bad, words = [], workspaces.status_words(device)
     for dev in {key[1] for key, _ in words}:
         torch.cuda.synchronize(dev)                  # a word may still be zeroed or raised on its own stream
